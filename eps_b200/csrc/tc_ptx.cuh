@@ -50,9 +50,11 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
-// Bounded wait.  Returns false when the CTA is aborting (this wait or another one gave up).
+// Bounded wait.  Returns false when the CTA is aborting (this wait or another one gave up).  The first try stands alone
+// in the instruction stream: in the steady state of a pipeline it succeeds, and the roles that are one thread have to
+// get through a K step in few instructions.
 template <class Storage>
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, Storage* sm, int32_t* status, int code) {
+__device__ __forceinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, Storage* sm, int32_t* status, int code) {
   uint64_t t0 = 0;
   uint32_t spins = 0;
   while (true) {
@@ -71,6 +73,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, Storag
       }
     }
   }
+}
+template <class Storage>
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, Storage* sm, int32_t* status, int code) {
+  if (__builtin_expect(mbar_try(bar, parity) != 0, 1)) return true;
+  return mbar_wait_slow(bar, parity, sm, status, code);
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -93,6 +100,15 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
+// One lane of a converged warp.  Producer and MMA warps run their loops with all lanes and let one issue: inside a branch on
+// the lane every operand of a TMA or MMA instruction has to be moved to a uniform register first (measured with the device
+// clock: 500 to 600 cycles to issue the loads of a stage, 250 this way; four MMAs and the commit 450 and 160).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r != 0;
+}
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
