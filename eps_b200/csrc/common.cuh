@@ -79,9 +79,9 @@ __device__ __forceinline__ uint16_t cvt_e4m3x2(float lo, float hi) {
   return r;
 }
 
-// The quantisation step shared by every producer of FP8 rows: clamp(x*inv, +-448) -> code.
-// fminf/fmaxf drop a NaN operand (0*inf for an all-zero group), as the reference relies on.
-__device__ __forceinline__ float quant_clamp(float x, float inv) { return fmaxf(-kFp8Max, fminf(x * inv, kFp8Max)); }
+// The quantisation step shared by every producer of FP8 rows: clamp(x*inv, +-448) -> code.  fminf drops a NaN operand
+// (0*inf for an all-zero group), as the reference relies on; the other side of the clamp is the saturation of cvt_e4m3x2.
+__device__ __forceinline__ float quant_clamp(float x, float inv) { return fminf(x * inv, kFp8Max); }
 
 template <bool kDivFull>
 __device__ __forceinline__ float scale_of_amax(float amax) {

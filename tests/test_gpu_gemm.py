@@ -89,6 +89,29 @@ def test_gemm_gateup_swiglu_requant(cuda, oracle, rows, I, K):
     assert np.all(np.abs(deq - act[:D]) <= bound)
 
 
+@pytest.mark.parametrize("rows", [[128], [7], [40, 200]])
+@pytest.mark.parametrize("gate_rms", [1e-3, 8.0, 60.0, 1e4])
+def test_gemm_gateup_over_the_range_of_the_activation(cuda, oracle, rows, gate_rms):
+    """Gates from the linear part of SiLU to far beyond where its exponential overflows, both orientations of a tile.
+    The group scales are amax/448 of the activations: fp32 sums in another order, here up to 512 terms of either sign
+    (2^-24 * 512 of the terms' magnitude, against an amax over 128 sums of them: below 1e-4), as is the activation."""
+    from eps_b200 import ops
+
+    I, K = 256, 512
+    rng = np.random.default_rng(len(rows))
+    excl, D, max_rows, A, a_s, B, b_s = _make(oracle, rng, rows, 2 * I, K)
+    b_s[:, :I // 128] *= np.float32(gate_rms / (0.02 * np.sqrt(K)))
+    q, s = ops.grouped_gemm_fp8(ops.GEMM_GATEUP, _dev(A, cuda), _dev(a_s, cuda), _dev(B, cuda), _dev(b_s, cuda),
+                                _dev(excl, cuda))
+    torch.cuda.synchronize()
+    act = oracle.swiglu(oracle.grouped_gemm_fp8(A, a_s, B, b_s, excl))[:D]
+    amax = np.abs(act).reshape(D, I // 128, 128).max(-1)
+    gq, gs = q.cpu().numpy()[:D], s.cpu().numpy()[:D]
+    assert np.all(np.isfinite(gs)) and np.all(np.abs(gs - amax / 448.0) <= 1e-4 * amax / 448.0)
+    deq = oracle.e4m3_table()[gq] * np.repeat(gs, 128, axis=1)
+    assert np.all(np.abs(deq - act) <= np.repeat(amax, 128, axis=1) * (2.0 ** -4) * 1.05)
+
+
 @pytest.mark.parametrize("rows,N,K", [([128], 256, 128), ([9, 250, 0, 40], 512, 1408 - 1408 % 128),
                                        ([130, 64, 33, 1, 161], 384, 256)])
 def test_gemm_down_weighted(cuda, oracle, rows, N, K):
