@@ -78,7 +78,8 @@ struct Storage {
   uint64_t tmem_empty[2];      // in a pair only the leader's are used: 8 epilogue warps of each CTA arrive
   uint32_t tmem_base;
   volatile int abort_flag;
-  int32_t tile_prefix[kMaxExperts + 1];
+  int32_t tile_prefix[kMaxExperts + 1];   // m-tiles before each expert
+  int32_t excl[kMaxExperts + 1];          // rows before each expert
 };
 
 // ---- cluster helpers of the paired form
@@ -118,6 +119,7 @@ struct Params {
   int32_t* status;
   int num_experts;
   int64_t N, K;
+  int kb;        // K / 64
   int n_tiles;
 };
 
@@ -136,11 +138,10 @@ __device__ __forceinline__ Tile locate(int t, const Params& p, const Storage<kCt
     if (sm->tile_prefix[mid] <= g) lo = mid;
     else hi = mid;
   }
-  c.e = lo;
-  const int m = g - sm->tile_prefix[lo];
-  const int b = __ldg(p.excl + lo), e_ = __ldg(p.excl + lo + 1);
-  c.row0 = b + m * kBM * kCtas;
-  c.rows_left = e_ - c.row0;
+  // from lane 0, so that the compiler knows them as warp-uniform (the operands of TMA and MMA instructions are)
+  c.e = __shfl_sync(0xffffffffu, lo, 0);
+  c.row0 = __shfl_sync(0xffffffffu, sm->excl[lo] + (g - sm->tile_prefix[lo]) * kBM * kCtas, 0);
+  c.rows_left = __shfl_sync(0xffffffffu, sm->excl[lo + 1], 0) - c.row0;
   return c;
 }
 
@@ -148,14 +149,18 @@ template <int kCtas>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                          const Params p) {
-  extern __shared__ uint8_t smem_raw[];
+  // Used as it stands (not through a rounded-up address), so that the compiler knows every access for one to shared
+  // memory; the swizzle needs the 1024-byte alignment, which the check makes sure of.
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   using St = Storage<kCtas>;
   constexpr int kStages = St::kStages;
-  St* sm = reinterpret_cast<St*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  St* sm = reinterpret_cast<St*>(smem_raw);
+  if ((smem_u32(smem_raw) & 1023u) != 0) {   // the same in every CTA
+    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, 51);
+    return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int KB = (int)(p.K / kBKElems);
   const uint32_t cta = kCtas == 2 ? cluster_ctarank() : 0u;   // 0 = the CTA that issues the MMAs
-  const int unit = (int)blockIdx.x / kCtas, units = (int)gridDim.x / kCtas;   // tiles are dealt to CTAs or to pairs
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -188,7 +193,12 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     for (int e0 = 0; e0 < p.num_experts; e0 += 32) {
       const int e = e0 + lane;
       int mt = 0;
-      if (e < p.num_experts) mt = (__ldg(p.excl + e + 1) - __ldg(p.excl + e) + kBM * kCtas - 1) / (kBM * kCtas);
+      if (e < p.num_experts) {
+        const int b = __ldg(p.excl + e), b1 = __ldg(p.excl + e + 1);
+        mt = (b1 - b + kBM * kCtas - 1) / (kBM * kCtas);
+        sm->excl[e] = b;
+        if (e + 1 == p.num_experts) sm->excl[e + 1] = b1;
+      }
       int inc = mt;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
@@ -204,79 +214,96 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   __syncthreads();
   if constexpr (kCtas == 2) cluster_sync_all();   // the peer's barriers exist before anything is sent to them
   tc_fence_after();
-  const uint32_t tmem_base = sm->tmem_base;
-  const int total_tiles = sm->tile_prefix[p.num_experts] * p.n_tiles;
-
+  // Tiles are dealt to CTAs or to pairs.  Every role reads what it needs here into its own registers; nothing computed
+  // before lives across the split.
+  auto first_tile = [&]() { return (int)blockIdx.x / kCtas; };
+  auto tile_step = [&]() { return (int)gridDim.x / kCtas; };
+  auto tile_count = [&]() { return sm->tile_prefix[p.num_experts] * p.n_tiles; };
   // 128 * dec + 256 * inc <= 384 * 168: setmaxnreg.inc blocks until the CTA's own register pool can serve it
   static_assert(128 * 40 + 256 * 232 <= kThreads * 168, "setmaxnreg budget exceeds the CTA's register pool");
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 0 && lane == 0) {
+    const int KB = p.kb, units = tile_step(), total_tiles = tile_count();
+    uint32_t stage = 0, phase = 0;   // place in the stage ring: the stage and the parity of its current round
+    auto next_stage = [&]() {
+      if (++stage == kStages) stage = 0, phase ^= 1u;
+    };
+    bool ok = true;
+    if (warp == 0) {
       // ------------------------------------------------ TMA producer (one per CTA).  In a pair each CTA loads its
       // own rows of A and its half of the weight rows; every copy reports its bytes to the LEADER's stage barrier,
       // on which the leader's producer has announced the bytes of both CTAs.
-      uint32_t it = 0;
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units) {
+      uint32_t full0 = 0;
+      if constexpr (kCtas == 2) full0 = map_to_cta(smem_u32(&sm->full[0]), 0);
+      for (int t = first_tile(); t < total_tiles && ok; t += units) {
         const Tile c = locate<kCtas>(t, p, sm);
         const int arow = c.row0 + kBM * (int)cta;
         const int brow = (int)(c.e * p.N + c.n * kBN) + (kBN / kCtas) * (int)cta;
-        for (int kb = 0; kb < KB; kb++, it++) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
-          if (!(ok = mbar_wait(&sm->empty[s], ph ^ 1, sm, p.status, 11))) break;
-          uint8_t* base = sm->tiles[s];
-          if constexpr (kCtas == 1) {
-            mbar_expect_tx(&sm->full[s], St::kStageBytes);
-            tma_load_2d(base, &tmap_a, kb * kBKElems, arow, &sm->full[s]);
-            tma_load_2d(base + kABytes, &tmap_b, kb * kBKElems, brow, &sm->full[s]);
-            tma_load_2d(base + 2 * kABytes, &tmap_b, kb * kBKElems, brow + 128, &sm->full[s]);
-          } else {
-            if (cta == 0) mbar_expect_tx(&sm->full[s], 2 * St::kStageBytes);
-            const uint32_t bar = map_to_cta(smem_u32(&sm->full[s]), 0);
-            tma_load_2d_pair(base, &tmap_a, kb * kBKElems, arow, bar);
-            tma_load_2d_pair(base + kABytes, &tmap_b, kb * kBKElems, brow, bar);
+        for (int kb = 0; kb < KB; kb++, next_stage()) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&sm->empty[stage], phase ^ 1u, sm, p.status, 11));
+          if (!ok) break;
+          uint8_t* base = sm->tiles[stage];
+          if (elect_one()) {
+            if constexpr (kCtas == 1) {
+              mbar_expect_tx(&sm->full[stage], St::kStageBytes);
+              tma_load_2d(base, &tmap_a, kb * kBKElems, arow, &sm->full[stage]);
+              tma_load_2d(base + kABytes, &tmap_b, kb * kBKElems, brow, &sm->full[stage]);
+              tma_load_2d(base + 2 * kABytes, &tmap_b, kb * kBKElems, brow + 128, &sm->full[stage]);
+            } else {
+              if (cta == 0) mbar_expect_tx(&sm->full[stage], 2 * St::kStageBytes);
+              const uint32_t bar = full0 + 8u * stage;
+              tma_load_2d_pair(base, &tmap_a, kb * kBKElems, arow, bar);
+              tma_load_2d_pair(base + kABytes, &tmap_b, kb * kBKElems, brow, bar);
+            }
           }
+          __syncwarp();
         }
       }
-      if (!ok) {
+      if (!ok && lane == 0) {
         const uint64_t t0 = global_ns();
         while (global_ns() - t0 < 200000ull) __nanosleep(1000);
       }
-    } else if (warp == 1 && lane == 0 && cta == 0) {
+    } else if (warp == 1 && cta == 0) {
       // ------------------------------------------------ MMA issuer (the leader's, for both CTAs of a pair)
       constexpr uint32_t idesc = bf16_idesc(kBM * kCtas, kBN);
-      uint32_t it = 0, tile_no = 0;
-      bool ok = true;
-      for (int t = unit; t < total_tiles && ok; t += units, tile_no++) {
-        const int buf = tile_no & 1;
-        const uint32_t tph = (tile_no >> 1) & 1;
-        if (!(ok = mbar_wait(&sm->tmem_empty[buf], tph ^ 1, sm, p.status, 21))) break;
-        const uint32_t d = tmem_base + (uint32_t)buf * kBN;
-        for (int kb = 0; kb < KB; kb++, it++) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
-          if (!(ok = mbar_wait(&sm->full[s], ph, sm, p.status, 22))) break;
+      const uint64_t da0 = smem_desc(smem_u32(sm->tiles[0])), db0 = smem_desc(smem_u32(sm->tiles[0]) + kABytes);
+      const uint32_t tmem_base = sm->tmem_base;
+      uint32_t empty_0 = 0, empty_1 = 0;
+      if constexpr (kCtas == 2) {
+        empty_0 = map_to_cta(smem_u32(&sm->empty[0]), 0);
+        empty_1 = map_to_cta(smem_u32(&sm->empty[0]), 1);
+      }
+      uint32_t tile_no = 0;
+      for (int t = first_tile(); t < total_tiles && ok; t += units, tile_no++) {
+        const uint32_t buf = tile_no & 1u;
+        ok = __all_sync(0xffffffffu, mbar_wait(&sm->tmem_empty[buf], ((tile_no >> 1) & 1u) ^ 1u, sm, p.status, 21));
+        if (!ok) break;
+        const uint32_t d = tmem_base + buf * kBN;
+        for (int kb = 0; kb < KB; kb++, next_stage()) {
+          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&sm->full[stage], phase, sm, p.status, 22)))) break;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sm->tiles[s]);
-          const uint64_t da = smem_desc(a_addr), db = smem_desc(a_addr + kABytes);
+          const uint64_t off = (uint64_t)(stage * (uint32_t)(St::kStageBytes >> 4));
+          const uint64_t da = da0 + off, db = db0 + off;
+          if (elect_one()) {
 #pragma unroll
-          for (int k4 = 0; k4 < 4; k4++)
-            umma_bf16<kCtas>(d, da + 2 * k4, db + 2 * k4, idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
-          if constexpr (kCtas == 1) {
-            umma_commit(&sm->empty[s]);
-          } else {   // the stage is free in both CTAs
-            umma_commit_pair(map_to_cta(smem_u32(&sm->empty[s]), 0));
-            umma_commit_pair(map_to_cta(smem_u32(&sm->empty[s]), 1));
+            for (int k4 = 0; k4 < 4; k4++)
+              umma_bf16<kCtas>(d, da + 2 * k4, db + 2 * k4, idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
+            if constexpr (kCtas == 1) {
+              umma_commit(&sm->empty[stage]);
+            } else {   // the stage is free in both CTAs
+              umma_commit_pair(empty_0 + 8u * stage);
+              umma_commit_pair(empty_1 + 8u * stage);
+            }
+            if (kb + 1 == KB) {
+              if constexpr (kCtas == 1) {
+                umma_commit(&sm->tmem_full[buf]);
+              } else {
+                umma_commit_pair(map_to_cta(smem_u32(&sm->tmem_full[buf]), 0));
+                umma_commit_pair(map_to_cta(smem_u32(&sm->tmem_full[buf]), 1));
+              }
+            }
           }
-        }
-        if (ok) {
-          if constexpr (kCtas == 1) {
-            umma_commit(&sm->tmem_full[buf]);
-          } else {
-            umma_commit_pair(map_to_cta(smem_u32(&sm->tmem_full[buf]), 0));
-            umma_commit_pair(map_to_cta(smem_u32(&sm->tmem_full[buf]), 1));
-          }
+          __syncwarp();
         }
       }
     }
@@ -285,10 +312,11 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     // ------------------------------------------------ epilogue: each CTA drains the accumulators of its own rows
     const int ew = warp - 4, quad = warp & 3, half = ew >> 2;
     const int r_in_tile = quad * 32 + lane;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const uint32_t lane_addr = sm->tmem_base + ((uint32_t)(quad * 32) << 16);
+    const int units = tile_step(), total_tiles = tile_count();
     uint32_t tile_no = 0;
     bool ok = true;
-    for (int t = unit; t < total_tiles && ok; t += units, tile_no++) {
+    for (int t = first_tile(); t < total_tiles && ok; t += units, tile_no++) {
       const Tile c = locate<kCtas>(t, p, sm);
       const int buf = tile_no & 1;
       ok = mbar_wait(&sm->tmem_full[buf], (tile_no >> 1) & 1u, sm, p.status, 31);
@@ -350,9 +378,9 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   if (warp == 1) {
     tc_fence_after();
     if constexpr (kCtas == 1)
-      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sm->tmem_base), "r"(kTmemCols) : "memory");
     else
-      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(sm->tmem_base), "r"(kTmemCols) : "memory");
   }
 }
 
@@ -398,7 +426,7 @@ namespace {
 template <int kCtas>
 int launch_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int64_t tiles_max, int sm_count,
                 cudaStream_t st) {
-  const size_t smem = sizeof(Storage<kCtas>) + 1024;
+  const size_t smem = sizeof(Storage<kCtas>);
   static std::atomic<int> max_units[64];   // per device: 0 = not configured yet, else CTAs (or pairs) that fit at once
   int dev = 0;
   cudaGetDevice(&dev);
@@ -478,6 +506,7 @@ extern "C" int epsb_grouped_gemm_bf16(const void* A, const void* B, const int32_
   p.num_experts = num_experts;
   p.N = N;
   p.K = K;
+  p.kb = (int)(K / kBKElems);
   p.n_tiles = (int)((N + kBN - 1) / kBN);
   // Pairs pay when the experts fill 256-row tiles (measured: +14 % at 512 and 1024 rows per expert, -6 % at
   // 300 +- 40 rows, where every expert's last pair tile is half empty); the row counts live on the device, so the
