@@ -1,6 +1,7 @@
 // Weighted row reductions of the combine path and the unfused SwiGLU (sm_100a).
 //
-// A warp owns an output row; each lane walks the row in 16-byte vectors (8 bf16)
+// A warp owns an output row, or one of `parts` interleaved parts of it when there are too few rows to fill the chip
+// (row_parts below); each lane walks it in 16-byte vectors (8 bf16)
 // and issues the loads of all summands of a vector before accumulating, so k
 // (or W) independent 16-byte loads per lane are in flight.  Two arithmetic
 // families are provided: "_ref" reproduces the reference kernels' bf16
@@ -69,7 +70,7 @@ template <bool kRefArith, int kSlots>
 __global__ void __launch_bounds__(kRedThreads)
 local_reduce_kernel(const uint8_t* __restrict__ y, const float* __restrict__ w_recv,
                     const int32_t* __restrict__ scale_map, const int32_t* __restrict__ red_map, StageWindows win,
-                    int k, int64_t H, uint8_t* __restrict__ send) {
+                    int k, int64_t H, int parts, uint8_t* __restrict__ send) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kRedWarps + (threadIdx.x >> 5);
   const int64_t n_warps = (int64_t)gridDim.x * kRedWarps;
@@ -81,7 +82,8 @@ local_reduce_kernel(const uint8_t* __restrict__ y, const float* __restrict__ w_r
     int64_t b, e;
     win.window(d, b, e);
     const int64_t first = (warp - seen % n_warps + n_warps) % n_warps;
-    for (int64_t q = b + first; q < e; q += n_warps) {
+    for (int64_t u = first; u < (e - b) * parts; u += n_warps) {
+      const int64_t q = b + u / parts;
       int32_t rows[kSlots];
       float wts[kSlots];
 #pragma unroll
@@ -96,7 +98,7 @@ local_reduce_kernel(const uint8_t* __restrict__ y, const float* __restrict__ w_r
           }
         }
       }
-      for (int v = lane; v < vecs; v += 32) {
+      for (int v = (int)(u % parts) * 32 + lane; v < vecs; v += 32 * parts) {
         uint4 in[kSlots];
 #pragma unroll
         for (int j = 0; j < kSlots; j++)
@@ -130,7 +132,7 @@ local_reduce_kernel(const uint8_t* __restrict__ y, const float* __restrict__ w_r
         st_16(send + q * row_bytes + (int64_t)v * 16, out);
       }
     }
-    seen += e - b;
+    seen += (e - b) * parts;
   }
 }
 
@@ -144,14 +146,15 @@ __global__ void __launch_bounds__(kRedThreads)
 reduce_ep1_kernel(const uint8_t* __restrict__ y, const int32_t* __restrict__ red_map,
                   const int32_t* __restrict__ glob_map, const int32_t* __restrict__ ret_incl, int S,
                   const uint8_t* __restrict__ shared, const uint8_t* __restrict__ x,
-                  const float* __restrict__ zero_scale, int T, int k, int64_t H, uint8_t* __restrict__ out) {
+                  const float* __restrict__ zero_scale, int T, int k, int64_t H, int parts, uint8_t* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kRedWarps + (threadIdx.x >> 5);
   const int64_t n_warps = (int64_t)gridDim.x * kRedWarps;
   const int vecs = (int)(H >> 3);
   const int64_t row_bytes = H * 2;
   const int64_t sentinel = (int64_t)ret_incl[S - 1] * k;
-  for (int64_t t = warp; t < T; t += n_warps) {
+  for (int64_t u = warp; u < (int64_t)T * parts; u += n_warps) {
+    const int64_t t = u / parts;
     const int32_t q = __ldg(glob_map + t);
     int32_t rows[kSlots];
 #pragma unroll
@@ -163,7 +166,7 @@ reduce_ep1_kernel(const uint8_t* __restrict__ y, const int32_t* __restrict__ red
       }
     }
     const float zs = zero_scale != nullptr ? __ldg(zero_scale + t) : 0.0f;
-    for (int v = lane; v < vecs; v += 32) {
+    for (int v = (int)(u % parts) * 32 + lane; v < vecs; v += 32 * parts) {
       const int64_t off = t * row_bytes + (int64_t)v * 16;
       uint4 in[kSlots];
 #pragma unroll
@@ -190,14 +193,15 @@ template <bool kRefArith, int kSlots>
 __global__ void __launch_bounds__(kRedThreads)
 global_reduce_kernel(const uint8_t* __restrict__ recv, const int32_t* __restrict__ glob_map,
                      const uint8_t* __restrict__ shared, const uint8_t* __restrict__ x,
-                     const float* __restrict__ zero_scale, int T, int W, int64_t H, uint8_t* __restrict__ out) {
+                     const float* __restrict__ zero_scale, int T, int W, int64_t H, int parts, uint8_t* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kRedWarps + (threadIdx.x >> 5);
   const int64_t n_warps = (int64_t)gridDim.x * kRedWarps;
   const int vecs = (int)(H >> 3);
   const int64_t row_bytes = H * 2;
   const int32_t sentinel = T * W;
-  for (int64_t t = warp; t < T; t += n_warps) {
+  for (int64_t u = warp; u < (int64_t)T * parts; u += n_warps) {
+    const int64_t t = u / parts;
     int32_t rows[kSlots];
 #pragma unroll
     for (int j = 0; j < kSlots; j++) {
@@ -208,7 +212,7 @@ global_reduce_kernel(const uint8_t* __restrict__ recv, const int32_t* __restrict
       }
     }
     const float zs = zero_scale != nullptr ? __ldg(zero_scale + t) : 0.0f;
-    for (int v = lane; v < vecs; v += 32) {
+    for (int v = (int)(u % parts) * 32 + lane; v < vecs; v += 32 * parts) {
       const int64_t off = t * row_bytes + (int64_t)v * 16;
       uint4 in[kSlots];
 #pragma unroll
@@ -266,16 +270,17 @@ template <bool kRefArith>
 __global__ void __launch_bounds__(kRedThreads)
 global_reduce_wide_kernel(const uint8_t* __restrict__ recv, const int32_t* __restrict__ glob_map,
                           const uint8_t* __restrict__ shared, const uint8_t* __restrict__ x,
-                          const float* __restrict__ zero_scale, int T, int W, int64_t H, uint8_t* __restrict__ out) {
+                          const float* __restrict__ zero_scale, int T, int W, int64_t H, int parts, uint8_t* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kRedWarps + (threadIdx.x >> 5);
   const int64_t n_warps = (int64_t)gridDim.x * kRedWarps;
   const int vecs = (int)(H >> 3);
   const int64_t row_bytes = H * 2;
   const int32_t sentinel = T * W;
-  for (int64_t t = warp; t < T; t += n_warps) {
+  for (int64_t u = warp; u < (int64_t)T * parts; u += n_warps) {
+    const int64_t t = u / parts;
     const float zs = zero_scale != nullptr ? __ldg(zero_scale + t) : 0.0f;
-    for (int v = lane; v < vecs; v += 32) {
+    for (int v = (int)(u % parts) * 32 + lane; v < vecs; v += 32 * parts) {
       const int64_t off = t * row_bytes + (int64_t)v * 16;
       BfVec acc;
       acc.u = make_uint4(0, 0, 0, 0);
@@ -326,13 +331,14 @@ template <int kSlots>
 __global__ void __launch_bounds__(kRedThreads)
 fastep_reduce_kernel(const uint8_t* __restrict__ rows_in, const uint8_t* __restrict__ raw,
                      const uint8_t* __restrict__ shared, const float* __restrict__ w,
-                     const int32_t* __restrict__ mapping, int T, int k, int64_t H, uint8_t* __restrict__ out) {
+                     const int32_t* __restrict__ mapping, int T, int k, int64_t H, int parts, uint8_t* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kRedWarps + (threadIdx.x >> 5);
   const int64_t n_warps = (int64_t)gridDim.x * kRedWarps;
   const int vecs = (int)(H >> 3);
   const int64_t row_bytes = H * 2;
-  for (int64_t t = warp; t < T; t += n_warps) {
+  for (int64_t u = warp; u < (int64_t)T * parts; u += n_warps) {
+    const int64_t t = u / parts;
     const uint8_t* srcs[kSlots];
     float wts[kSlots];
 #pragma unroll
@@ -345,7 +351,7 @@ fastep_reduce_kernel(const uint8_t* __restrict__ rows_in, const uint8_t* __restr
         wts[j] = __ldg(w + t * k + j);
       }
     }
-    for (int v = lane; v < vecs; v += 32) {
+    for (int v = (int)(u % parts) * 32 + lane; v < vecs; v += 32 * parts) {
       uint4 in[kSlots];
 #pragma unroll
       for (int j = 0; j < kSlots; j++)
@@ -365,7 +371,7 @@ fastep_reduce_kernel(const uint8_t* __restrict__ rows_in, const uint8_t* __restr
 
 __global__ void __launch_bounds__(kRedThreads)
 silu_kernel(const uint8_t* __restrict__ gate_up, uint8_t* __restrict__ act, const int32_t* __restrict__ bounds,
-            int num_experts, int64_t rows, int64_t I) {
+            int num_experts, int64_t rows, int64_t I, int parts) {
   int64_t begin = 0, end = rows;
   if (bounds != nullptr) {
     begin = bounds[0];
@@ -375,10 +381,11 @@ silu_kernel(const uint8_t* __restrict__ gate_up, uint8_t* __restrict__ act, cons
   const int64_t warp = (int64_t)blockIdx.x * kRedWarps + (threadIdx.x >> 5);
   const int64_t n_warps = (int64_t)gridDim.x * kRedWarps;
   const int vecs = (int)(I >> 3);
-  for (int64_t r = begin + warp; r < end; r += n_warps) {
+  for (int64_t q = warp; q < (end - begin) * parts; q += n_warps) {
+    const int64_t r = begin + q / parts;
     const uint8_t* g = gate_up + r * I * 4;
     const uint8_t* u = g + I * 2;
-    for (int v = lane; v < vecs; v += 32) {
+    for (int v = (int)(q % parts) * 32 + lane; v < vecs; v += 32 * parts) {
       const uint4 gv = ld_nc_16(g + (int64_t)v * 16), uv = ld_nc_16(u + (int64_t)v * 16);
       const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, uw[4] = {uv.x, uv.y, uv.z, uv.w};
       uint32_t ow[4];
@@ -403,6 +410,15 @@ silu_kernel(const uint8_t* __restrict__ gate_up, uint8_t* __restrict__ act, cons
     else if ((n) <= 12) { constexpr int kS = 12; __VA_ARGS__; } \
     else { constexpr int kS = 16; __VA_ARGS__; }                \
   } while (0)
+
+// Parts of a row of H bf16: 1 where the rows alone fill every SM with warps, else as many as do, down to one 16-byte vector
+// per lane.  A warp alone walks a 7168-wide row with 8 summands in 28 dependent steps of one memory latency: 128 rows took
+// 36 us undivided (0.5 TB/s) where the bytes need 3.
+int row_parts(int64_t rows, int64_t H) {
+  const int64_t steps = (H / 8 + 31) / 32;
+  const int64_t want = (int64_t)sm_count() * 8 * kRedWarps / (rows > 0 ? rows : 1);
+  return (int)(want < 1 ? 1 : (want > steps ? steps : want));
+}
 
 int red_grid(int64_t rows) {
   int64_t want = (rows + kRedWarps - 1) / kRedWarps;
@@ -432,8 +448,9 @@ extern "C" int epsb_local_reduce_ref(const void* y, const float* w_recv, const i
   EPSB_REQUIRE(stage >= -1 && stage < S, EPSB_ERR_INVALID, "stage %d out of range for %d stages", stage, S);
   if (max_rows <= 0) return EPSB_OK;
   StageWindows win{ret_incl, W, S, stage};
-  EPSB_SLOT_SWITCH(k, (local_reduce_kernel<true, kS><<<red_grid(max_rows), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      (const uint8_t*)y, w_recv, scale_map, red_map, win, k, H, (uint8_t*)send)));
+  const int parts = row_parts(stage < 0 ? max_rows : (max_rows + S - 1) / S, H);   // a stage covers about 1/S of the rows
+  EPSB_SLOT_SWITCH(k, (local_reduce_kernel<true, kS><<<red_grid(max_rows * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      (const uint8_t*)y, w_recv, scale_map, red_map, win, k, H, parts, (uint8_t*)send)));
   return check_launch("local_reduce_ref");
 }
 
@@ -445,8 +462,9 @@ extern "C" int epsb_local_reduce(const void* y, const int32_t* red_map, const in
   EPSB_REQUIRE(stage >= -1 && stage < S, EPSB_ERR_INVALID, "stage %d out of range for %d stages", stage, S);
   if (max_rows <= 0) return EPSB_OK;
   StageWindows win{ret_incl, W, S, stage};
-  EPSB_SLOT_SWITCH(k, (local_reduce_kernel<false, kS><<<red_grid(max_rows), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      (const uint8_t*)y, nullptr, nullptr, red_map, win, k, H, (uint8_t*)send)));
+  const int parts = row_parts(stage < 0 ? max_rows : (max_rows + S - 1) / S, H);   // a stage covers about 1/S of the rows
+  EPSB_SLOT_SWITCH(k, (local_reduce_kernel<false, kS><<<red_grid(max_rows * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      (const uint8_t*)y, nullptr, nullptr, red_map, win, k, H, parts, (uint8_t*)send)));
   return check_launch("local_reduce");
 }
 
@@ -459,13 +477,14 @@ static int launch_global_reduce(const void* recv, const int32_t* glob_map, const
   EPSB_REQUIRE(zero_scale == nullptr || x != nullptr, EPSB_ERR_INVALID, "zero_scale needs the raw input x");
   if (T <= 0) return EPSB_OK;
   auto st = static_cast<cudaStream_t>(stream);
+  const int parts = row_parts(T, H);
   if (W <= kMaxSlots)
-    EPSB_SLOT_SWITCH(W, (global_reduce_kernel<kRef, kS><<<red_grid(T), kRedThreads, 0, st>>>(
-        (const uint8_t*)recv, glob_map, (const uint8_t*)shared, (const uint8_t*)x, zero_scale, T, W, H, (uint8_t*)out)));
+    EPSB_SLOT_SWITCH(W, (global_reduce_kernel<kRef, kS><<<red_grid((int64_t)T * parts), kRedThreads, 0, st>>>(
+        (const uint8_t*)recv, glob_map, (const uint8_t*)shared, (const uint8_t*)x, zero_scale, T, W, H, parts, (uint8_t*)out)));
   else
-    global_reduce_wide_kernel<kRef><<<red_grid(T), kRedThreads, 0, st>>>((const uint8_t*)recv, glob_map,
+    global_reduce_wide_kernel<kRef><<<red_grid((int64_t)T * parts), kRedThreads, 0, st>>>((const uint8_t*)recv, glob_map,
                                                                          (const uint8_t*)shared, (const uint8_t*)x,
-                                                                         zero_scale, T, W, H, (uint8_t*)out);
+                                                                         zero_scale, T, W, H, parts, (uint8_t*)out);
   return check_launch("global_reduce");
 }
 
@@ -488,9 +507,10 @@ extern "C" int epsb_reduce_ep1(const void* y, const int32_t* red_map, const int3
   EPSB_REQUIRE(S > 0, EPSB_ERR_INVALID, "num_stages %d", S);
   EPSB_REQUIRE(zero_scale == nullptr || x != nullptr, EPSB_ERR_INVALID, "zero_scale needs the raw input x");
   if (T <= 0) return EPSB_OK;
-  EPSB_SLOT_SWITCH(k, (reduce_ep1_kernel<kS><<<red_grid(T), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  const int parts = row_parts(T, H);
+  EPSB_SLOT_SWITCH(k, (reduce_ep1_kernel<kS><<<red_grid((int64_t)T * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       (const uint8_t*)y, red_map, glob_map, ret_incl, S, (const uint8_t*)shared, (const uint8_t*)x, zero_scale, T, k, H,
-      (uint8_t*)out)));
+      parts, (uint8_t*)out)));
   return check_launch("reduce_ep1");
 }
 
@@ -500,8 +520,9 @@ extern "C" int epsb_fastep_reduce(const void* rows, const void* raw, const void*
   if (rc) return rc;
   EPSB_REQUIRE(k > 0 && k <= kMaxSlots, EPSB_ERR_INVALID, "topk %d exceeds %d", k, kMaxSlots);
   if (T <= 0) return EPSB_OK;
-  EPSB_SLOT_SWITCH(k, (fastep_reduce_kernel<kS><<<red_grid(T), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      (const uint8_t*)rows, (const uint8_t*)raw, (const uint8_t*)shared, w, mapping, T, k, H, (uint8_t*)out)));
+  const int parts = row_parts(T, H);
+  EPSB_SLOT_SWITCH(k, (fastep_reduce_kernel<kS><<<red_grid((int64_t)T * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      (const uint8_t*)rows, (const uint8_t*)raw, (const uint8_t*)shared, w, mapping, T, k, H, parts, (uint8_t*)out)));
   return check_launch("fastep_reduce");
 }
 
@@ -510,7 +531,8 @@ extern "C" int epsb_silu_run(const void* gate_up, void* act, const int32_t* excl
   EPSB_REQUIRE(inter_size > 0 && inter_size % 8 == 0, EPSB_ERR_INVALID, "Unsupported inter_size: %lld",
                (long long)inter_size);
   if (rows <= 0) return EPSB_OK;
-  silu_kernel<<<red_grid(rows), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      (const uint8_t*)gate_up, (uint8_t*)act, exclusive_sum, num_experts, rows, inter_size);
+  const int parts = row_parts(rows, inter_size);
+  silu_kernel<<<red_grid(rows * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      (const uint8_t*)gate_up, (uint8_t*)act, exclusive_sum, num_experts, rows, inter_size, parts);
   return check_launch("silu_run");
 }

@@ -271,3 +271,45 @@ def test_reduce_ep1_matches_two_pass_semantics(cuda, oracle, T, k, H, S, shared,
             acc = (x[t].float().numpy().astype(np.float64) * np.float64(zs[t].item()) + acc.astype(np.float64)).astype(np.float32)
         want[t] = acc
     assert np.array_equal(_bits(out), oracle.bf16_bits(want))
+
+
+@pytest.mark.parametrize("H", [8, 264, 2304])
+def test_a_rows_sum_does_not_depend_on_how_many_rows_there_are(cuda, H):
+    """Few rows are divided over several warps each, many are not (the line lies at the warps the chip holds): the same
+    bits on both sides of it and at every division."""
+    from eps_b200 import ops
+
+    T, k = 9480, 4
+    g = torch.Generator().manual_seed(H)
+    rows = torch.randn((2 * T, H), generator=g).to(torch.bfloat16).to(cuda)
+    raw = torch.randn((T, H), generator=g).to(torch.bfloat16).to(cuda)
+    w = torch.rand((T, k), generator=g).to(cuda)
+    mapping = torch.randint(0, 2 * T, (T, k), generator=g, dtype=torch.int32).to(cuda)
+    full = ops.fastep_reduce(rows, raw, w, mapping.view(-1), torch.empty((T, H), dtype=torch.bfloat16, device=cuda))
+    want = (rows.float()[mapping.long()] * w.unsqueeze(2)).sum(dim=1)
+    assert torch.all((full.float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5)   # one bf16 rounding, fp32 sums of 4
+    for n in (1, 3, 700, 3158, 4736, 9472):
+        part = ops.fastep_reduce(rows, raw, w[:n].contiguous(), mapping[:n].contiguous().view(-1),
+                                 torch.empty((n, H), dtype=torch.bfloat16, device=cuda))
+        assert torch.equal(part, full[:n]), n
+
+
+@pytest.mark.parametrize("n_seg", [1, 255, 256, 257, 1024, 1100])
+def test_arrange_rows_segment_counts(cuda, n_seg):
+    """Segments of 0 to 5 rows, copied to another order, around the number of segments a CTA scans at a time."""
+    from eps_b200 import ops
+
+    g = torch.Generator().manual_seed(n_seg)
+    rows = torch.randint(0, 6, (n_seg,), generator=g)
+    src_off = rows.cumsum(0) - rows
+    perm = torch.randperm(n_seg, generator=g)
+    dst_off = torch.empty_like(rows)
+    dst_off[perm] = rows[perm].cumsum(0) - rows[perm]
+    n = int(rows.sum())
+    src = torch.randint(0, 256, (max(n, 1), 48), generator=g, dtype=torch.uint8)
+    want = torch.full_like(src, 7)
+    for s in range(n_seg):
+        want[dst_off[s]:dst_off[s] + rows[s]] = src[src_off[s]:src_off[s] + rows[s]]
+    dst = torch.full_like(src, 7).to(cuda)
+    ops.arrange_rows(src.to(cuda), dst, *(t.int().to(cuda) for t in (src_off, rows, dst_off)), n_seg, max(n, 1))
+    assert torch.equal(dst.cpu(), want)
