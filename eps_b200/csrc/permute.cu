@@ -82,26 +82,60 @@ scatter_rows_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, 
   }
 }
 
-// Segments are handed to CTAs round-robin in chunks of rows so that one long
-// segment does not serialise on a single CTA.
+// The rows of all segments, concatenated, are dealt to the warps of the grid one by one, so that one long segment does not
+// serialise on a few warps.  Every CTA scans the row counts of up to kArrangeSegs segments at a time in shared memory; a
+// warp finds a row's segment there by bisection.  (Each warp walking the whole list with a 64-bit remainder per segment
+// took 245 us for 256 segments of 128 rows x 14 KB, 3.8 TB/s; this 160, 5.9 TB/s.)
+constexpr int kArrangeSegs = 4 * kMoveThreads;
+
 __global__ void __launch_bounds__(kMoveThreads)
 arrange_rows_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, const int32_t* __restrict__ src_off,
                     const int32_t* __restrict__ rows, const int32_t* __restrict__ dst_off, int n_seg,
                     int64_t row_bytes) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t)blockIdx.x * kMoveWarps + (threadIdx.x >> 5);
-  const int64_t n_warps = (int64_t)gridDim.x * kMoveWarps;
+  __shared__ int32_t first[kArrangeSegs + 1];   // rows before each segment of this batch
+  __shared__ int32_t warp_sum[kMoveWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int n_warps = (int)gridDim.x * kMoveWarps;
   const int vecs = (int)(row_bytes >> 4);
-  // Every warp walks the segment list; row r of the concatenation goes to warp r % n_warps.
-  int64_t seen = 0;
-  for (int p = 0; p < n_seg; p++) {
-    const int64_t nr = __ldg(rows + p);
-    const int64_t so = __ldg(src_off + p), d_o = __ldg(dst_off + p);
-    int64_t first = (warp - seen % n_warps + n_warps) % n_warps;
-    for (int64_t i = first; i < nr; i += n_warps)
-      copy_row(reinterpret_cast<const uint4*>(src + (so + i) * row_bytes),
-               reinterpret_cast<uint4*>(dst + (d_o + i) * row_bytes), vecs, lane);
-    seen += nr;
+  int64_t seen = 0;   // rows of earlier batches
+  for (int s0 = 0; s0 < n_seg; s0 += kArrangeSegs) {
+    const int n = min(kArrangeSegs, n_seg - s0);
+    int v[4], sum = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int s = threadIdx.x * 4 + i;
+      v[i] = sum;
+      sum += s < n ? __ldg(rows + s0 + s) : 0;
+    }
+    int inc = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += o;
+    }
+    __syncthreads();   // the previous batch's prefix is no longer read
+    if (lane == 31) warp_sum[w] = inc;
+    __syncthreads();
+    int before = inc - sum;
+    for (int i = 0; i < w; i++) before += warp_sum[i];
+#pragma unroll
+    for (int i = 0; i < 4; i++) first[threadIdx.x * 4 + i] = before + v[i];
+    if (threadIdx.x == kMoveThreads - 1) first[kArrangeSegs] = before + sum;
+    __syncthreads();
+    const int total = first[kArrangeSegs];
+    const int turn = (int)(seen % n_warps), me = (int)blockIdx.x * kMoveWarps + w;
+    for (int i = me >= turn ? me - turn : me - turn + n_warps; i < total; i += n_warps) {
+      int lo = 0, hi = n;   // the segment with first[lo] <= i < first[lo + 1]
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= i) lo = mid;
+        else hi = mid;
+      }
+      const int r = i - first[lo];
+      copy_row(reinterpret_cast<const uint4*>(src + ((int64_t)__ldg(src_off + s0 + lo) + r) * row_bytes),
+               reinterpret_cast<uint4*>(dst + ((int64_t)__ldg(dst_off + s0 + lo) + r) * row_bytes), vecs, lane);
+    }
+    seen += total;
   }
 }
 
