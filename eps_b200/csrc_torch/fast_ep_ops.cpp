@@ -37,6 +37,15 @@ class FastEP {
   void dispatch(int32_t* out_exclusive_sum, void* out_expert_x, int64_t out_rows, const void* dp_x,
                 const int32_t* indices, int64_t T, cudaStream_t st) {
     if (T * k_ > rows_) throw std::runtime_error("tokens exceed max_num_global_tokens");
+    if (W_ == 1 && !overlap(out_expert_x, out_rows, dp_x, T)) {
+      // the rows' order is final as it is sent: straight into the caller's buffer, no exchange, no regrouping
+      raise_if(epsb_fastep_expand_plan(indices, (int)T, k_, E_, out_exclusive_sum, mapping_.data_ptr<int32_t>(), st));
+      if (T > 0) raise_if(epsb_scatter_rows(dp_x, out_expert_x, mapping_.data_ptr<int32_t>(), k_, T * k_, H_ * 2, st));
+      dp_x_ = dp_x;
+      T_ = T;
+      dispatched_ = true;
+      return;
+    }
     raise_if(epsb_fastep_expand_plan(indices, (int)T, k_, E_, excl_.data_ptr<int32_t>(), mapping_.data_ptr<int32_t>(), st));
     if (T > 0) raise_if(epsb_scatter_rows(dp_x, send_.data_ptr(), mapping_.data_ptr<int32_t>(), k_, T * k_, H_ * 2, st));
     if (W_ == 1) {
@@ -67,6 +76,16 @@ class FastEP {
   void combine(void* out_tokens, const float* weights, const void* expert_y, int64_t y_rows, const void* shared,
                cudaStream_t st) {
     if (!dispatched_) throw std::runtime_error("combine called before dispatch");
+    if (W_ == 1) {   // the expert's rows lie where the reduction looks for them
+      if (overlap(out_tokens, T_, expert_y, y_rows)) {
+        const int64_t n = std::min(y_rows, rows_);
+        cuda_ok(cudaMemcpyAsync(send_.data_ptr(), expert_y, (size_t)(n * H_ * 2), cudaMemcpyDeviceToDevice, st), "copy");
+        expert_y = send_.data_ptr();
+      }
+      raise_if(epsb_fastep_reduce(expert_y, dp_x_, shared, weights, mapping_.data_ptr<int32_t>(), (int)T_, k_, H_,
+                                  out_tokens, st));
+      return;
+    }
     int32_t* pl = plan_.data_ptr<int32_t>();
     const int64_t pitch = plan_.size(1);
     // inverse regroup: [expert][source] -> [source][expert] in the receive buffer of dispatch
@@ -79,6 +98,11 @@ class FastEP {
   }
 
  private:
+  bool overlap(const void* a, int64_t a_rows, const void* b, int64_t b_rows) const {
+    const char *pa = static_cast<const char*>(a), *pb = static_cast<const char*>(b);
+    return pa < pb + b_rows * H_ * 2 && pb < pa + a_rows * H_ * 2;
+  }
+
   void windows() {
     send_begin_.assign(W_, 0); send_end_.assign(W_, 0); recv_begin_.assign(W_, 0); recv_end_.assign(W_, 0);
     const int64_t* dummy = nullptr;

@@ -16,6 +16,12 @@ from ._lib import EpsError
 from .communication import Communicator
 
 
+def _overlap(a: torch.Tensor, b: torch.Tensor) -> bool:
+    """Whether two contiguous tensors share memory."""
+    return (a.data_ptr() < b.data_ptr() + b.numel() * b.element_size()
+            and b.data_ptr() < a.data_ptr() + a.numel() * a.element_size())
+
+
 class AllToAll:
     def __init__(self, top_k: int, num_experts: int, hidden_size: int, max_num_global_tokens: int,
                  comm: Communicator | None, dtype: torch.dtype = torch.bfloat16, device=None) -> None:
@@ -41,6 +47,13 @@ class AllToAll:
         W, EL = self.W, self.EL
         if T * self.k > self.rows:
             raise EpsError("tokens exceed max_num_global_tokens")
+        if W == 1 and not _overlap(out_expert_x, dp_x):
+            # The rows' order is final as it is sent: straight into the caller's buffer, no exchange, no regrouping.
+            _, mapping = ops.fastep_expand_plan(indices, self.E, excl=out_exclusive_sum)
+            if T > 0:
+                ops.scatter_rows(dp_x, out_expert_x, mapping, self.k, T * self.k)
+            self.ctx = dict(T=T, mapping=mapping, dp_x=dp_x, arr=None, host=None)
+            return
         excl, mapping = ops.fastep_expand_plan(indices, self.E)
         if T > 0:
             ops.scatter_rows(dp_x, self.send, mapping, self.k, T * self.k)
@@ -69,12 +82,20 @@ class AllToAll:
         if c is None:
             raise EpsError("combine called before dispatch")
         W, EL = self.W, self.EL
+        if W == 1:
+            rows = expert_y   # they lie where the reduction looks for them
+            if _overlap(out_tokens, expert_y):
+                n = min(expert_y.shape[0], self.rows)
+                rows = self.send
+                rows[:n].copy_(expert_y[:n])
+            ops._check(rows, "expert_y")
+            ops.fastep_reduce(rows, c["dp_x"], weights, c["mapping"], out_tokens, shared=shared)
+            return
         arr_src, arr_rows, arr_dst = c["arr"]
         # inverse regroup: [expert][source] -> [source][expert] in the return-send buffer (the receive buffer of dispatch)
         ops.arrange_rows(expert_y, self.recv, arr_dst, arr_rows, arr_src, EL * W, expert_y.shape[0])
-        if W > 1:
-            send_b, send_e, recv_b, recv_e, _ = c["host"]
-            # what I received from p goes back to p and lands where p sent it from
-            self.comm.exchange([self.recv[int(a):int(b)] for a, b in zip(recv_b, recv_e)],
-                               [self.send[int(a):int(b)] for a, b in zip(send_b, send_e)])
+        send_b, send_e, recv_b, recv_e, _ = c["host"]
+        # what I received from p goes back to p and lands where p sent it from
+        self.comm.exchange([self.recv[int(a):int(b)] for a, b in zip(recv_b, recv_e)],
+                           [self.send[int(a):int(b)] for a, b in zip(send_b, send_e)])
         ops.fastep_reduce(self.send, c["dp_x"], weights, c["mapping"], out_tokens, shared=shared)

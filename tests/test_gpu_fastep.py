@@ -44,6 +44,34 @@ def test_fastep_roundtrip_single_rank(cuda, oracle, T, k, E, H, nz):
     assert np.array_equal(_bits(out), want)
 
 
+def test_fastep_buffers_that_share_memory(cuda, oracle):
+    """The expert rows may be written over the tokens and the output over the expert rows, as with separate buffers."""
+    from eps_b200.fast_ep import AllToAll
+
+    T, k, E, H = 40, 4, 8, 256
+    idx, w = random_routing(np.random.default_rng(5), T, k, E, 0)
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(cuda)
+    idx, w = torch.from_numpy(idx).to(cuda), torch.from_numpy(w).to(cuda)
+    excl = torch.empty((E + 1,), dtype=torch.int32, device=cuda)
+
+    def run(rows, tokens, out):
+        a2a = AllToAll(k, E, H, T, None)
+        a2a.dispatch(excl, rows, tokens, idx, T)
+        got = rows.clone()
+        tokens = tokens if out is None else x
+        out = torch.empty_like(x) if out is None else out
+        a2a.combine(out, w, rows, T)
+        return got, out.clone()
+
+    rows = torch.zeros((T * k, H), dtype=torch.bfloat16, device=cuda)
+    want_rows, want_out = run(rows, x, None)
+    shared = torch.zeros((T * k, H), dtype=torch.bfloat16, device=cuda)
+    shared[:T] = x
+    assert torch.equal(run(shared, shared[:T], None)[0], want_rows)
+    rows.zero_()
+    assert torch.equal(run(rows, x, rows[:T])[1], want_out)
+
+
 def test_executor_classes(cuda, oracle):
     from eps_b200._lib import EpsError
     from eps_b200.executor import AokGroupedGemm, silu
