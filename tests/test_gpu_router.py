@@ -162,3 +162,18 @@ def test_router_errors(cuda):
         ops.topk_sigmoid(s, None, 3, 2, 2)            # 3 groups do not divide 64
     with pytest.raises(EpsError):
         ops.topk_sigmoid(s, None, 4, 1, 17)           # top-17 out of one group of 16
+
+
+@pytest.mark.parametrize("E,g,tg,k", [(64, 1, 1, 5), (64, 8, 3, 12), (32, 32, 6, 4), (1024, 32, 32, 32)])
+def test_router_ties_go_to_the_lower_id(cuda, E, g, tg, k):
+    """Equal scores everywhere (and, with one expert per group, group scores that are all the sentinel): groups and
+    experts in ascending order of their ids, whichever lanes hold them; a single larger score still comes first."""
+    from eps_b200 import ops
+
+    logits = torch.zeros((2, E))
+    logits[1, k - 1] = 3.0
+    idx, w = ops.topk_sigmoid(logits.to(cuda), None, g, tg, k, 1.0)
+    want = list(range(k))
+    assert idx[0].tolist() == want
+    assert idx[1].tolist() == [k - 1] + want[:k - 1]
+    assert torch.allclose(w[0].cpu(), torch.full((k,), 1.0 / k), rtol=1e-6)
