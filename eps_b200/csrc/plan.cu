@@ -127,7 +127,8 @@ __device__ __forceinline__ int strided_order(int v, int n, int NT) {
 //   void skip(int pos, int j)          called once per sub-item with key < 0
 // Positions 0..n_pos-1 are already in visiting order.  On return s.base/s.total
 // hold the exclusive bucket offsets and the bucket sizes.
-template <class P>
+// kLast: nothing in the kernel reads what this sort emits to global memory.
+template <bool kLast, class P>
 __device__ void stable_bucket_sort(P& p, int n_pos, int B, SortScratch s, uint16_t* key_cache = nullptr) {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
@@ -144,7 +145,9 @@ __device__ void stable_bucket_sort(P& p, int n_pos, int B, SortScratch s, uint16
   const int chunk = ((n_items + C * kPlanThreads - 1) / (C * kPlanThreads)) * 32;
   const int cta_begin = min(n_items, crank * kPlanWarps * chunk);
   const int i_begin = min(n_items, (crank * kPlanWarps + warp) * chunk), i_end = min(n_items, i_begin + chunk);
-  for (int i = threadIdx.x; i < kPlanWarps * B; i += kPlanThreads) s.rows[i] = 0;
+  // warps of this CTA that own items: the rows of the others are neither cleared nor scanned
+  const int used = min(kPlanWarps, chunk > 0 ? (max(0, n_items - cta_begin) + chunk - 1) / chunk : 0);
+  for (int i = threadIdx.x; i < used * B; i += kPlanThreads) s.rows[i] = 0;
   __syncthreads();
   int32_t* my_row = s.rows + warp * B;
   for (int i0 = i_begin; i0 < i_end; i0 += 32 * kKeyUnroll) {
@@ -152,7 +155,7 @@ __device__ void stable_bucket_sort(P& p, int n_pos, int B, SortScratch s, uint16
 #pragma unroll
     for (int u = 0; u < kKeyUnroll; u++) {
       const int i = i0 + u * 32 + lane;
-      keys[u] = i < i_end ? p.key(i / J, i % J) : -1;
+      keys[u] = i < i_end ? (J == 1 ? p.key(i, 0) : p.key(i / J, i % J)) : -1;
     }
 #pragma unroll
     for (int u = 0; u < kKeyUnroll; u++) {
@@ -170,15 +173,15 @@ __device__ void stable_bucket_sort(P& p, int n_pos, int B, SortScratch s, uint16
   for (int b = threadIdx.x; b < B; b += kPlanThreads) {
     int run = 0;
 #pragma unroll 8
-    for (int w = 0; w < kPlanWarps; w++) {
+    for (int w = 0; w < used; w++) {
       const int c = s.rows[w * B + b];
       s.rows[w * B + b] = run;
       run += c;
     }
     s.ltotal[b] = run;
   }
-  cluster.sync();  // every CTA's bucket totals are in its shared memory
-  for (int b = threadIdx.x; b < B; b += kPlanThreads) {
+  if (C > 1) cluster.sync();  // every CTA's bucket totals are in its shared memory
+  for (int b = threadIdx.x; b < B; b += kPlanThreads) {   // (the same thread wrote this CTA's)
     int before = 0, all = 0;
     for (int c = 0; c < C; c++) {
       const int v = c == crank ? s.ltotal[b] : cluster.map_shared_rank(s.ltotal, c)[b];
@@ -202,7 +205,7 @@ __device__ void stable_bucket_sort(P& p, int n_pos, int B, SortScratch s, uint16
       const int i = i0 + u * 32 + lane;
       if (i >= i_end) keys[u] = -1;
       else if (key_cache != nullptr) keys[u] = key_cache[i - cta_begin] == 0xffffu ? -1 : (int)key_cache[i - cta_begin];
-      else keys[u] = p.key(i / J, i % J);
+      else keys[u] = J == 1 ? p.key(i, 0) : p.key(i / J, i % J);
     }
 #pragma unroll
     for (int u = 0; u < kKeyUnroll; u++) {
@@ -216,16 +219,21 @@ __device__ void stable_bucket_sort(P& p, int n_pos, int B, SortScratch s, uint16
         if (key >= 0 && (m & lt_mask) == 0) my_row[key] += __popc(m);
         __syncwarp();
         if (i < i_end) {
-          if (key >= 0) p.emit(i / J, i % J, mine);
-          else p.skip(i / J, i % J);
+          const int pos = J == 1 ? i : i / J, j = J == 1 ? 0 : i - pos * J;
+          if (key >= 0) p.emit(pos, j, mine);
+          else p.skip(pos, j);
         }
       }
     }
   }
   // What the CTAs emitted to global memory is visible to the whole cluster, and nobody reads this CTA's
   // bucket totals any more, once every CTA is past this point.
-  __threadfence();
-  cluster.sync();
+  if (C > 1) {
+    if (!kLast) __threadfence();
+    cluster.sync();
+  } else {
+    __syncthreads();
+  }
 }
 
 // Thread index and thread count of the whole cluster, for the element-wise loops around the sorts.
@@ -254,12 +262,14 @@ struct CommPlanProblem {
   __device__ int token(int pos) const { return strided_order(pos, T, NT); }
   __device__ int key(int pos, int ep) const {
     const int32_t* row = idx + (size_t)token(pos) * k;
+    const int first = ep * EL;   // experts [first, first + EL) are rank ep's
     int lead = INT32_MAX;
+#pragma unroll 4
     for (int j = 0; j < k; j++) {
       const int e = row[j];
-      if (e >= 0 && e / EL == ep) lead = min(lead, e % EL);
+      if (e >= first && e < first + EL) lead = min(lead, e);
     }
-    return lead == INT32_MAX ? -1 : ep * EL + lead;
+    return lead == INT32_MAX ? -1 : lead;
   }
   __device__ void emit(int pos, int ep, int out) const { send_map[out] = ep * T + token(pos); }
   __device__ void skip(int, int) const {}
@@ -275,12 +285,14 @@ struct GlobalPlanProblem {
     const int m = send_map[pos];
     const int ep = m / T, t = m % T;
     const int32_t* row = idx + (size_t)t * k;
+    const int first = ep * EL;
     int tail = -1;
+#pragma unroll 4
     for (int j = 0; j < k; j++) {
       const int e = row[j];
-      if (e >= 0 && e / EL == ep) tail = max(tail, e % EL);
+      if (e >= first && e < first + EL) tail = max(tail, e);
     }
-    return tail < 0 ? -1 : ep * EL + tail;
+    return tail;
   }
   __device__ void emit(int pos, int, int out) const {
     const int m = send_map[pos];
@@ -297,9 +309,13 @@ source_plans_kernel(const int32_t* __restrict__ idx, const float* __restrict__ w
   const int EL = E / W;
   SortScratch s = carve(plan_smem, E);
   uint16_t* cache = cache_after(plan_smem, E, cache_items);
+  // (before the first sort, whose last barrier makes the fill of glob_map visible to the cluster)
+  if (glob_map != nullptr)
+    for (int i = cluster_tid(); i < T * W; i += cluster_threads()) glob_map[i] = T * W;
   if (zero_scale != nullptr && weights != nullptr) {
     for (int t = cluster_tid(); t < T; t += cluster_threads()) {
       float z = 0.0f;
+#pragma unroll 4
       for (int j = 0; j < k; j++)
         if (idx[(size_t)t * k + j] < 0) z += weights[(size_t)t * k + j];
       zero_scale[t] = z;
@@ -308,15 +324,13 @@ source_plans_kernel(const int32_t* __restrict__ idx, const float* __restrict__ w
   int NT = (T + 15) / 16;
   NT = max(1, min(NT, 128));
   CommPlanProblem cp{idx, send_map, T, k, W, EL, NT};
-  stable_bucket_sort(cp, T, E, s, cache);
+  stable_bucket_sort<false>(cp, T, E, s, cache);
   write_stage_sums(s, W, EL, S, send_incl);
   if (glob_map == nullptr) return;
   const int n_sent = s.base[E - 1] + s.total[E - 1];
-  for (int i = cluster_tid(); i < T * W; i += cluster_threads()) glob_map[i] = T * W;
-  __threadfence();
-  cg::this_cluster().sync();  // the glob_map fill (and, from the sort above, send_map) is visible to the cluster
   GlobalPlanProblem gp{idx, send_map, glob_map, T, k, W, EL};
-  stable_bucket_sort(gp, n_sent, E, s, cache);
+  __syncthreads();   // the first sort's bucket sums have been read
+  stable_bucket_sort<true>(gp, n_sent, E, s, cache);
   write_stage_sums(s, W, EL, S, coll_incl);
 }
 
@@ -391,6 +405,7 @@ struct LocalReducePlanProblem {
     int dp = 0;
     while (dp < W - 1 && r >= recv_incl[dp * S + S - 1]) dp++;
     int tail = -1;
+#pragma unroll 4
     for (int j = 0; j < k; j++) {
       const int g = ridx[(size_t)r * k + j];
       if (lo <= g && g < hi) tail = max(tail, g - lo);
@@ -399,6 +414,7 @@ struct LocalReducePlanProblem {
   }
   __device__ void emit(int r, int, int out) const {
     scale_map[out] = r;
+#pragma unroll 4
     for (int j = 0; j < k; j++) red_map[(size_t)out * k + j] = inv_gemm[(size_t)r * k + j];
   }
   __device__ void skip(int, int) const {}
@@ -431,7 +447,7 @@ expert_plans_kernel(const int32_t* __restrict__ ridx, const int32_t* __restrict_
   {
     SortScratch s = carve(plan_smem, EL);
     GemmPlanProblem gp{ridx, gemm_map, inv_gemm, R, k, lo, hi, NT};
-    stable_bucket_sort(gp, R, EL, s, cache);
+    stable_bucket_sort<false>(gp, R, EL, s, cache);
     if (cluster_leader()) {
       for (int e = threadIdx.x; e < EL; e += kPlanThreads) excl[e + 1] = s.base[e] + s.total[e];
       if (threadIdx.x == 0) excl[0] = 0;
@@ -441,7 +457,7 @@ expert_plans_kernel(const int32_t* __restrict__ ridx, const int32_t* __restrict_
   __syncthreads();  // inv_gemm is complete and visible (the sort ended with a cluster-wide fence and barrier)
   SortScratch s = carve(plan_smem, W * EL);
   LocalReducePlanProblem lp{ridx, recv_incl, inv_gemm, scale_map, red_map, k, lo, hi, W, S, EL};
-  stable_bucket_sort(lp, R, W * EL, s, cache);
+  stable_bucket_sort<true>(lp, R, W * EL, s, cache);
   write_stage_sums(s, W, EL, S, ret_incl);
 }
 
@@ -471,7 +487,7 @@ fastep_expand_plan_kernel(const int32_t* __restrict__ idx, int T, int k, int E, 
   extern __shared__ int32_t plan_smem[];
   SortScratch s = carve(plan_smem, E);
   FastEpExpandProblem fp{idx, mapping, s.base, s.total, k};
-  stable_bucket_sort(fp, T, E, s);
+  stable_bucket_sort<true>(fp, T, E, s);
   if (!cluster_leader()) return;
   for (int e = threadIdx.x; e < E; e += kPlanThreads) excl[e + 1] = s.base[e] + s.total[e];
   if (threadIdx.x == 0) excl[0] = 0;
@@ -551,7 +567,7 @@ oep_arrange_plan_kernel(const int32_t* __restrict__ ids, int n, int32_t size_per
   extern __shared__ int32_t plan_smem[];
   SortScratch s = carve(plan_smem, W);
   OepArrangeProblem op{ids, mapping, send_map, size_per_rank, W};
-  stable_bucket_sort(op, n, W, s);
+  stable_bucket_sort<true>(op, n, W, s);
   if (!cluster_leader()) return;
   for (int r = threadIdx.x; r < W; r += kPlanThreads) send_incl[r] = s.base[r] + s.total[r];
 }
