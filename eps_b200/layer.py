@@ -133,14 +133,17 @@ class MoELayerFP8:
         if self.W == 1:
             # nothing is staged: the GEMM reads the quantised tokens through the composed plans
             sched.context.raw_input = x
-            a_rows, row_w, src_h, src_s = sched.gemm_sources(expert_weights, xq, xs)
-            n += 1
+            if self.gemm_gathers_rows:
+                a_rows, row_w, src_h, src_s = sched.gemm_sources(expert_weights, xq, xs)
+                n += 1
+            else:
+                row_w = torch.empty((D,), dtype=torch.float32, device=self.dev)
         else:
             sched.prologue(expert_weights, xq, xs, None if self.direct_sources else self.A_s[:D], raw_input=x,
                            defer_exchange=True)
             # NCCL transport: gate weights, hidden rows, scales to send order; scales to GEMM order; GEMM-row gate
-            # weights.  Device-side exchange: nothing is staged, only the per-GEMM-row sources.
-            n += 1 if self.direct_sources else 5
+            # weights.  Device-side exchange: nothing is staged.
+            n += (1 if self.gemm_gathers_rows else 0) if self.direct_sources else 5
             row_w = None
         eps_ = EL // S
 
@@ -154,10 +157,8 @@ class MoELayerFP8:
                                      self.wgu_s[s * eps_:(s + 1) * eps_], ex, out=self.act[:D],
                                      out_scales=self.act_s[:D], status=self.status, a_rows=a_rows[:D])
             else:
-                if self.direct_sources:   # one gather from the source rows into expert order (rows and their scales)
-                    b0, b1 = s * eps_, (s + 1) * eps_
-                    ops.gather_rows(src_h, self.A[:D], a_rows, 1, ops.INT32_MAX, bounds=excl, b0=b0, b1=b1)
-                    ops.gather_rows(src_s, self.A_s[:D], a_rows, 1, ops.INT32_MAX, bounds=excl, b0=b0, b1=b1)
+                if self.direct_sources:   # one gather from the source rows into expert order
+                    sched.gather_gemm_rows(expert_weights, xq, xs, self.A[:D], self.A_s[:D], row_w, s)
                 ops.grouped_gemm_fp8(ops.GEMM_GATEUP, self.A[:D], self.A_s[:D], self.wgu[s * eps_:(s + 1) * eps_],
                                      self.wgu_s[s * eps_:(s + 1) * eps_], ex, out=self.act[:D],
                                      out_scales=self.act_s[:D], status=self.status)
@@ -170,7 +171,7 @@ class MoELayerFP8:
         if self.W == 1:
             for s in range(S):
                 stage_gemms(s)
-                n += 2 if self.gemm_gathers_rows else 4
+                n += 2 if self.gemm_gathers_rows else 3
         else:
             # Stage pipeline on two streams (the reference leaves this to its caller): all dispatches are queued on
             # the communication stream up front, each combine as soon as its stage has been reduced, so the exchange
@@ -191,8 +192,10 @@ class MoELayerFP8:
             for s in range(S):
                 main.wait_event(disp_done[s])
                 if s == 0:  # the first dispatch carried the gate weights and the input scales
-                    if self.direct_sources:
+                    if self.direct_sources and self.gemm_gathers_rows:
                         a_rows, row_w, src_h, src_s = sched.gemm_sources(expert_weights, xq, xs)
+                    elif self.direct_sources:
+                        row_w = torch.empty((D,), dtype=torch.float32, device=self.dev)
                     else:
                         sched.finish_prologue()
                         row_w = sched.gemm_row_weights()
@@ -208,7 +211,7 @@ class MoELayerFP8:
                     mark = self._exchange_mark("combine", s, comm_stream) if sched.peer is None else None
                     sched.combine(s)
                     self._exchange_done(mark, comm_stream)
-                n += 4 if (self.gemm_gathers_rows or not self.direct_sources) else 6
+                n += 4 if (self.gemm_gathers_rows or not self.direct_sources) else 5
             all_back = torch.cuda.Event()
             all_back.record(comm_stream)
         if self.W > 1:

@@ -309,6 +309,21 @@ def gemm_row_sources(gemm_map, excl, num_experts, k, max_rows, w_src=None, send_
     return a_rows, row_w
 
 
+def gather_gemm_rows(hidden, scales, gemm_map, excl, e0, e1, k, max_rows, A, A_s, row_w=None, w_src=None, send_map=None,
+                     T=0):
+    """The rows of experts [e0, e1) in GEMM order with their scales and gate weights: gemm_row_sources and the gathers of
+    hidden rows and scales in one pass (rows of A / A_s / row_w outside the experts' range are not written)."""
+    _check(hidden, "hidden")
+    _check(scales, "scales")
+    _check(A, "A")
+    _check(A_s, "A_s")
+    if _row_bytes(hidden) != _row_bytes(A) or _row_bytes(scales) != _row_bytes(A_s):
+        raise EpsError("source and GEMM rows differ in size")
+    call("epsb_gather_gemm_rows", ptr(hidden), _row_bytes(hidden), ptr(scales), _row_bytes(scales) // 4, ptr(gemm_map),
+         ptr(excl), int(e0), int(e1), int(k), ptr(send_map), int(T), ptr(w_src), max_rows, ptr(A), ptr(A_s), ptr(row_w),
+         stream_ptr())
+
+
 def grouped_gemm_fp8(mode, A, a_s, B, b_s, excl, out=None, out_scales=None, row_w=None, status=None,
                      sm_count=0, a_rows=None):
     """FP8 block-scaled grouped GEMM; see include/eps_b200.h for the three modes.

@@ -525,6 +525,23 @@ class Scheduler:
         a_rows, row_w = ops.gemm_row_sources(ctx.gemm_map, ctx.excl, EL, k, n, w_src=self.recv_w)
         return a_rows, row_w, self.recv_hidden, self.recv_scales
 
+    def gather_gemm_rows(self, expert_scales: torch.Tensor, hidden: torch.Tensor, scales: torch.Tensor, A: torch.Tensor,
+                         A_s: torch.Tensor, row_w: torch.Tensor, stage_idx: int) -> None:
+        """The stage's GEMM rows in expert order, with their scales and gate weights: what `gemm_sources` and two row
+        gathers through its result give, in one launch.  In a world of one the rows come from the caller's `hidden` /
+        `scales` / `expert_scales`, otherwise from the receive arena."""
+        ctx = self.context
+        EL, k = self.local_num_experts, self.top_k
+        eps_ = EL // ctx.num_stages
+        n = max(ctx.rows_bound, 0) * min(k, EL)
+        T, send_map, w_src = 0, None, self.recv_w
+        if self.W == 1:
+            T, send_map, w_src = ctx.num_tokens, ctx.send_map if ctx.num_tokens > 0 else None, expert_scales
+        else:
+            hidden, scales = self.recv_hidden, self.recv_scales
+        ops.gather_gemm_rows(hidden, scales, ctx.gemm_map, ctx.excl, stage_idx * eps_, (stage_idx + 1) * eps_, k, n, A, A_s,
+                             row_w=row_w, w_src=w_src, send_map=send_map, T=T)
+
     # helper used by the fused layer
     def gemm_row_weights(self) -> torch.Tensor:
         ctx = self.context

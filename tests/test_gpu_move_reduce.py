@@ -313,3 +313,30 @@ def test_arrange_rows_segment_counts(cuda, n_seg):
     dst = torch.full_like(src, 7).to(cuda)
     ops.arrange_rows(src.to(cuda), dst, *(t.int().to(cuda) for t in (src_off, rows, dst_off)), n_seg, max(n, 1))
     assert torch.equal(dst.cpu(), want)
+
+
+@pytest.mark.parametrize("T,k,EL,H,stages,with_map", [(1, 1, 1, 128, 1, True), (37, 4, 8, 1408, 2, True), (300, 6, 16, 2560, 4, False), (9, 8, 32, 7168, 1, True)])
+def test_gather_gemm_rows_equals_sources_and_two_gathers(cuda, T, k, EL, H, stages, with_map):
+    from eps_b200 import ops
+
+    g = torch.Generator().manual_seed(T + H)
+    idx = torch.stack([torch.randperm(EL, generator=g)[:k] for _ in range(T)]) if k <= EL else None
+    pairs = sorted((int(e), t * k + j) for t in range(T) for j, e in enumerate(idx[t].tolist()))
+    gemm_map = torch.tensor([m for _, m in pairs], dtype=torch.int32, device=cuda)
+    counts = torch.bincount(idx.reshape(-1), minlength=EL)
+    excl = torch.cat([torch.zeros(1, dtype=torch.int64), counts.cumsum(0)]).int().to(cuda)
+    D = T * k
+    hidden = torch.randint(0, 256, (T, H), generator=g, dtype=torch.uint8).to(cuda)
+    scales, w = torch.rand((T, H // 128), generator=g).to(cuda), torch.rand((T, k), generator=g).to(cuda)
+    send_map = torch.randperm(T, generator=g).int().to(cuda) if with_map else None
+    a_rows, row_w = ops.gemm_row_sources(gemm_map, excl, EL, k, D, w_src=w, send_map=send_map, T=T if with_map else 0)
+    want = ops.gather_rows(hidden, torch.zeros((D, H), dtype=torch.uint8, device=cuda), a_rows)
+    want_s = ops.gather_rows(scales, torch.zeros((D, H // 128), device=cuda), a_rows)
+    A, A_s = torch.full_like(want, 7), torch.full_like(want_s, -1.0)
+    got_w = torch.full((D,), -1.0, device=cuda)
+    for s in range(stages):
+        ops.gather_gemm_rows(hidden, scales, gemm_map, excl, s * EL // stages, (s + 1) * EL // stages, k, D, A, A_s,
+                             row_w=got_w, w_src=w, send_map=send_map, T=T if with_map else 0)
+        end = int(excl[(s + 1) * EL // stages])
+        assert torch.all(A[end:] == 7) and torch.all(A_s[end:] == -1.0)
+    assert torch.equal(A, want) and torch.equal(A_s, want_s) and torch.equal(got_w, row_w)
