@@ -125,21 +125,6 @@ struct RingPos {
   }
 };
 
-// x * sigmoid(x), a tenth of a gate/up tile's time.  exp(-x) as 2^t with the rounding error of t = -x * log2(e) put back to
-// first order (the plain 2^fl(t) is off by up to |x| ulp), then the approximate reciprocal.  Relative error against 64 bits
-// (rms over uniform x): |x| <= 4 5.4e-8, <= 16 5.5e-8, <= 60 4.8e-8; with __expf and a correctly rounded reciprocal, in about
-// twice the instructions, 6.3e-8, 1.9e-7 and 7.2e-7.
-__device__ __forceinline__ float silu(float x) {
-  constexpr float kL2eHi = 1.44269502162933349609375f, kL2eLo = 1.92596299112661746e-8f, kLn2 = 0.693147180559945f;
-  const float t = x * -kL2eHi;
-  const float r = fmaf(x, -kL2eLo, fmaf(x, -kL2eHi, -t));
-  float e, q;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
-  if (fabsf(t) < 128.0f) e = fmaf(e, r * kLn2, e);   // (beyond, e is 0 or inf and r may be anything)
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(1.0f + e));
-  return x * q;
-}
-
 // Epilogue of a tail tile (see kTailMax).  TMEM lanes = the 128 weight rows of a block, columns [0, T) = block 0
 // (gate rows, or the tile's first 128 weight rows), [T, 2T) = block 1 (up rows, or the second 128), T = 2 * kTh.
 // The warp of quadrant `quad` and column half `half` owns weight rows 32*quad + lane and tokens
@@ -212,7 +197,7 @@ __device__ __forceinline__ bool tail_tile(const GemmParams& p, Storage* sm, cons
 #pragma unroll
     for (int i = 0; i < kTh; i++) {
       const float g = acc0[i], u = acc1[i];
-      const float a = silu(g) * u;
+      const float a = (g * __frcp_rn(1.0f + __expf(-g))) * u;
       acc0[i] = a;
       // |a| of a finite float orders like its bit pattern; a NaN (only in token columns past the expert's
       // rows, never stored) may win the maximum there and nowhere else
@@ -541,7 +526,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ AMaps tmap_a, const __grid_const
 #pragma unroll
         for (int i = 0; i < 64; i++) {
           const float g = acc[i], u = acc[64 + i];
-          const float a = silu(g) * u;   // checked by tolerance, not bit-exact
+          const float a = (g * __frcp_rn(1.0f + __expf(-g))) * u;  // silu(g) * u; checked by tolerance, not bit-exact
           acc[i] = a;
           amax = fmaxf(amax, fabsf(a));
         }

@@ -94,22 +94,62 @@ def test_gemm_gateup_swiglu_requant(cuda, oracle, rows, I, K):
 def test_gemm_gateup_over_the_range_of_the_activation(cuda, oracle, rows, gate_rms):
     """Gates from the linear part of SiLU to far beyond where its exponential overflows, both orientations of a tile.
     The group scales are amax/448 of the activations: fp32 sums in another order, here up to 512 terms of either sign
-    (2^-24 * 512 of the terms' magnitude, against an amax over 128 sums of them: below 1e-4), as is the activation."""
+    (2^-24 * 512 of the terms' magnitude, against an amax over 128 sums of them: below 1e-4), as is the activation.
+    Every element is then off by that and by its own e4m3 rounding: 2^-4 of itself, 2^-10 of the scale for subnormal codes."""
     from eps_b200 import ops
 
     I, K = 256, 512
     rng = np.random.default_rng(len(rows))
     excl, D, max_rows, A, a_s, B, b_s = _make(oracle, rng, rows, 2 * I, K)
     b_s[:, :I // 128] *= np.float32(gate_rms / (0.02 * np.sqrt(K)))
+    status = torch.zeros(4, dtype=torch.int32, device=cuda)
     q, s = ops.grouped_gemm_fp8(ops.GEMM_GATEUP, _dev(A, cuda), _dev(a_s, cuda), _dev(B, cuda), _dev(b_s, cuda),
-                                _dev(excl, cuda))
+                                _dev(excl, cuda), status=status)
     torch.cuda.synchronize()
+    _check_status(status)
     act = oracle.swiglu(oracle.grouped_gemm_fp8(A, a_s, B, b_s, excl))[:D]
     amax = np.abs(act).reshape(D, I // 128, 128).max(-1)
     gq, gs = q.cpu().numpy()[:D], s.cpu().numpy()[:D]
     assert np.all(np.isfinite(gs)) and np.all(np.abs(gs - amax / 448.0) <= 1e-4 * amax / 448.0)
     deq = oracle.e4m3_table()[gq] * np.repeat(gs, 128, axis=1)
-    assert np.all(np.abs(deq - act) <= np.repeat(amax, 128, axis=1) * (2.0 ** -4) * 1.05)
+    sums = 1e-4 * np.repeat(amax, 128, axis=1)
+    assert np.all(np.abs(deq - act) <= 2.0 ** -4 * (np.abs(act) + sums) + 2.0 ** -10 * np.repeat(gs, 128, axis=1) + sums)
+
+
+@pytest.mark.parametrize("rows", [128, 40, 7])
+def test_gemm_gateup_activation_in_every_binade(cuda, oracle, rows):
+    """One product an output and powers of two around it, so that gate and up are exact and the group scale is
+    |silu(g) * u| / 448 alone, against 64 bits.  u = 2^60 * g keeps the activation a normal number down to gates of -88.6,
+    where the reciprocal of 1 + exp(-g) is subnormal already.  The bound is the arithmetic's: exp(-g) within
+    2 + 1.173 |g| ulp, and five roundings of half an ulp (1 + e, reciprocal, two products, the scale), an ulp being 2^-23;
+    a subnormal reciprocal is a multiple of 2^-149."""
+    from eps_b200 import ops
+
+    I, K = 128, 128
+    g = np.concatenate([-np.linspace(88.6, 86.0, 40), -np.geomspace(86.0, 1e-3, 40), np.geomspace(1e-3, 400.0, 48)])
+    g = g.astype(np.float32)[np.random.default_rng(3).permutation(128)]
+    E = 128 // rows
+    g = g[:E * rows]
+    one = int(np.flatnonzero(oracle.e4m3_table() == 1.0)[0])
+    A, B = np.zeros((E * rows, K), dtype=np.uint8), np.zeros((E, 2 * I, K), dtype=np.uint8)
+    A[:, 5] = one
+    B[:, :, 5] = one
+    b_s = np.ones((E, 2, 1), dtype=np.float32)
+    b_s[:, 1] = 2.0 ** 60
+    excl = np.arange(E + 1, dtype=np.int32) * rows
+    status = torch.zeros(4, dtype=torch.int32, device=cuda)
+    q, s = ops.grouped_gemm_fp8(ops.GEMM_GATEUP, _dev(A, cuda), _dev(g[:, None], cuda), _dev(B, cuda), _dev(b_s, cuda),
+                                _dev(excl, cuda), status=status)
+    torch.cuda.synchronize()
+    _check_status(status)
+    g64 = g.astype(np.float64)
+    sig = 1.0 / (1.0 + np.exp(-g64))
+    want = np.abs(g64 * sig * (g64 * 2.0 ** 60)) / 448.0
+    rel = 2.0 ** -23 * (2.0 + 1.173 * np.abs(g64) + 2.5) + 2.0 ** -149 / sig
+    got = s.cpu().numpy()[:, 0]
+    assert np.all(np.abs(got - want) <= rel * want), (g[np.argmax(np.abs(got - want) / want)], np.max(np.abs(got / want - 1)))
+    top = int(np.flatnonzero(oracle.e4m3_table() == 448.0)[0])   # silu(g) * g is positive: every code of a row is its top one
+    assert np.all(q.cpu().numpy() == top)
 
 
 @pytest.mark.parametrize("rows,N,K", [([128], 256, 128), ([9, 250, 0, 40], 512, 1408 - 1408 % 128),
