@@ -428,6 +428,8 @@ int red_grid(int64_t rows) {
   return (int)want;
 }
 
+bool vec_aligned(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
 int check_h(int64_t H) {
   EPSB_REQUIRE(H > 0 && H % 8 == 0, EPSB_ERR_INVALID, "hidden size %lld is not a multiple of 8", (long long)H);
   return EPSB_OK;
@@ -519,7 +521,11 @@ extern "C" int epsb_fastep_reduce(const void* rows, const void* raw, const void*
   int rc = check_h(H);
   if (rc) return rc;
   EPSB_REQUIRE(k > 0 && k <= kMaxSlots, EPSB_ERR_INVALID, "topk %d exceeds %d", k, kMaxSlots);
+  // `rows` may be a caller's own tensor, and a view into a larger one may start anywhere
+  EPSB_REQUIRE(vec_aligned(rows), EPSB_ERR_INVALID, "row buffers must be 16-byte aligned");
   if (T <= 0) return EPSB_OK;
+  EPSB_REQUIRE(vec_aligned(raw) && vec_aligned(shared) && vec_aligned(out), EPSB_ERR_INVALID,
+               "row buffers must be 16-byte aligned");
   const int parts = row_parts(T, H);
   EPSB_SLOT_SWITCH(k, (fastep_reduce_kernel<kS><<<red_grid((int64_t)T * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       (const uint8_t*)rows, (const uint8_t*)raw, (const uint8_t*)shared, w, mapping, T, k, H, parts, (uint8_t*)out)));

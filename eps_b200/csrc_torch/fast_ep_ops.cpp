@@ -34,13 +34,15 @@ class FastEP {
     plan_ = at::empty({5, std::max(EL_ * W_, W_ + 1)}, dev.dtype(at::kInt));
   }
 
+  int64_t hidden() const { return H_; }
+
   void dispatch(int32_t* out_exclusive_sum, void* out_expert_x, int64_t out_rows, const void* dp_x,
                 const int32_t* indices, int64_t T, cudaStream_t st) {
     if (T * k_ > rows_) throw std::runtime_error("tokens exceed max_num_global_tokens");
-    if (W_ == 1 && !overlap(out_expert_x, out_rows, dp_x, T)) {
+    if (W_ == 1 && out_rows > 0 && !overlap(out_expert_x, out_rows, dp_x, T)) {
       // the rows' order is final as it is sent: straight into the caller's buffer, no exchange, no regrouping
       raise_if(epsb_fastep_expand_plan(indices, (int)T, k_, E_, out_exclusive_sum, mapping_.data_ptr<int32_t>(), st));
-      if (T > 0) raise_if(epsb_scatter_rows(dp_x, out_expert_x, mapping_.data_ptr<int32_t>(), k_, T * k_, H_ * 2, st));
+      raise_if(epsb_scatter_rows(dp_x, out_expert_x, mapping_.data_ptr<int32_t>(), k_, T * k_, H_ * 2, st));
       dp_x_ = dp_x;
       T_ = T;
       dispatched_ = true;
@@ -77,7 +79,8 @@ class FastEP {
                cudaStream_t st) {
     if (!dispatched_) throw std::runtime_error("combine called before dispatch");
     if (W_ == 1) {   // the expert's rows lie where the reduction looks for them
-      if (overlap(out_tokens, T_, expert_y, y_rows)) {
+      if (reinterpret_cast<uintptr_t>(expert_y) % 16 != 0) throw std::runtime_error("row buffers must be 16-byte aligned");
+      if (y_rows == 0 || overlap(out_tokens, T_, expert_y, y_rows)) {
         const int64_t n = std::min(y_rows, rows_);
         cuda_ok(cudaMemcpyAsync(send_.data_ptr(), expert_y, (size_t)(n * H_ * 2), cudaMemcpyDeviceToDevice, st), "copy");
         expert_y = send_.data_ptr();
@@ -179,6 +182,8 @@ void combine(fptr_t ptr, at::Tensor& outTokens, const at::Tensor& weights, const
   check(weights, 2, "weights");
   TORCH_CHECK(weights.scalar_type() == at::kFloat, "weights must be of type Float32");
   check(expertY, 2, "expertY");
+  TORCH_CHECK(expertY.size(1) * expertY.element_size() == fe(ptr)->hidden() * 2, "expertY must have rows of ",
+              fe(ptr)->hidden() * 2, " bytes");
   fe(ptr)->combine(outTokens.data_ptr(), weights.data_ptr<float>(), expertY.data_ptr(), expertY.size(0), nullptr,
                    current_stream());
 }

@@ -47,11 +47,10 @@ class AllToAll:
         W, EL = self.W, self.EL
         if T * self.k > self.rows:
             raise EpsError("tokens exceed max_num_global_tokens")
-        if W == 1 and not _overlap(out_expert_x, dp_x):
+        if W == 1 and out_expert_x.shape[0] > 0 and not _overlap(out_expert_x, dp_x):
             # The rows' order is final as it is sent: straight into the caller's buffer, no exchange, no regrouping.
             _, mapping = ops.fastep_expand_plan(indices, self.E, excl=out_exclusive_sum)
-            if T > 0:
-                ops.scatter_rows(dp_x, out_expert_x, mapping, self.k, T * self.k)
+            ops.scatter_rows(dp_x, out_expert_x, mapping, self.k, T * self.k)
             self.ctx = dict(T=T, mapping=mapping, dp_x=dp_x, arr=None, host=None)
             return
         excl, mapping = ops.fastep_expand_plan(indices, self.E)
@@ -83,12 +82,16 @@ class AllToAll:
             raise EpsError("combine called before dispatch")
         W, EL = self.W, self.EL
         if W == 1:
+            ops._check(expert_y, "expert_y", dim=2)
+            if ops._row_bytes(expert_y) != ops._row_bytes(self.send):
+                raise EpsError(f"expert_y must have rows of {ops._row_bytes(self.send)} bytes")
+            if expert_y.data_ptr() % 16:
+                raise EpsError("row buffers must be 16-byte aligned")
             rows = expert_y   # they lie where the reduction looks for them
-            if _overlap(out_tokens, expert_y):
+            if expert_y.shape[0] == 0 or _overlap(out_tokens, expert_y):
                 n = min(expert_y.shape[0], self.rows)
                 rows = self.send
-                rows[:n].copy_(expert_y[:n])
-            ops._check(rows, "expert_y")
+                rows[:n].view(torch.uint8).copy_(expert_y[:n].view(torch.uint8))
             ops.fastep_reduce(rows, c["dp_x"], weights, c["mapping"], out_tokens, shared=shared)
             return
         arr_src, arr_rows, arr_dst = c["arr"]

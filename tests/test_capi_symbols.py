@@ -42,6 +42,19 @@ def test_argument_validation_needs_no_gpu():
         call("epsb_grouped_gemm_fp8", 0, None, None, None, None, None, 4, 16, 128, 100, None, None, None, None, 0, None)
 
 
+def test_fastep_reduce_refuses_misaligned_rows():
+    """Its rows may be a caller's view into a larger tensor; 16-byte loads from an odd address would fault on the device, so
+    the host refuses it (the addresses here are made up: nothing is launched)."""
+    import pytest
+
+    from eps_b200._lib import EpsError, call
+
+    a = 1 << 20
+    for rows, raw, shared, out in [(a + 2, a, None, a), (a, a + 8, None, a), (a, a, a + 4, a), (a, a, a, a + 14)]:
+        with pytest.raises(EpsError, match="row buffers must be 16-byte aligned"):
+            call("epsb_fastep_reduce", rows, raw, shared, a, a, 4, 2, 256, out, None)
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     import pytest
 

@@ -72,6 +72,40 @@ def test_fastep_buffers_that_share_memory(cuda, oracle):
     assert torch.equal(run(rows, x, rows[:T])[1], want_out)
 
 
+def test_fastep_combine_refuses_rows_it_cannot_read(cuda):
+    """expert_y is read where it lies: a misaligned view, other row sizes and strided rows are refused on the host, also
+    where the output shares its memory; no rows at all are fine as long as none is asked for."""
+    from eps_b200._lib import EpsError
+    from eps_b200.fast_ep import AllToAll
+
+    T, k, E, H = 6, 2, 4, 64
+    idx = torch.arange(T * k, dtype=torch.int32, device=cuda).view(T, k) % E
+    w = torch.full((T, k), 0.5, device=cuda)
+    x = torch.ones((T, H), dtype=torch.bfloat16, device=cuda)
+    excl = torch.empty((E + 1,), dtype=torch.int32, device=cuda)
+    a2a = AllToAll(k, E, H, T, None)
+    a2a.dispatch(excl, torch.empty((T * k, H), dtype=torch.bfloat16, device=cuda), x, idx, T)
+    out = torch.empty_like(x)
+    flat = torch.ones((T * k * H + 8,), dtype=torch.bfloat16, device=cuda)
+    odd = flat[1:1 + T * k * H].view(T * k, H)
+    for target in (out, flat[1:1 + T * H].view(T, H)):
+        with pytest.raises(EpsError, match="16-byte aligned"):
+            a2a.combine(target, w, odd, T)
+    for bad in (torch.ones((T * k, 2 * H), dtype=torch.bfloat16, device=cuda), torch.ones((T * k, H), device=cuda)):
+        with pytest.raises(EpsError, match="rows of 128 bytes"):
+            a2a.combine(out, w, bad, T)
+    with pytest.raises(EpsError, match="contiguous"):
+        a2a.combine(out, w, torch.ones((T * k, 2 * H), dtype=torch.bfloat16, device=cuda)[:, :H], T)
+    a2a.combine(out, w, flat[8:].view(T * k, H), T)
+    assert torch.equal(out, x)
+    idx.fill_(-1)   # identity experts only: no expert row exists
+    none = torch.empty((0, H), dtype=torch.bfloat16, device=cuda)
+    a2a.dispatch(excl, none, x, idx, T)
+    out.zero_()
+    a2a.combine(out, w, none, T)
+    assert torch.equal(out, x) and not bool(excl.any())
+
+
 def test_executor_classes(cuda, oracle):
     from eps_b200._lib import EpsError
     from eps_b200.executor import AokGroupedGemm, silu

@@ -339,6 +339,46 @@ def test_fast_ep_ops_bit_exact(cuda, oracle, eps_pkg):
 
 
 @pytest.mark.gpu
+def test_fast_ep_ops_buffers_that_share_memory(cuda, eps_pkg):
+    """Expert rows over the tokens, and the output over the expert rows, as with separate buffers; views that the combine
+    cannot read with 16-byte loads and rows of another size are refused on the host."""
+    from eps.fast_ep import AllToAll
+    from helpers import random_routing
+
+    T, k, E, H = 40, 4, 8, 256
+    idx, w = random_routing(np.random.default_rng(5), T, k, E, 2)
+    x = torch.randn((T, H), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(cuda)
+    idx, w = torch.from_numpy(idx).to(cuda), torch.from_numpy(w).to(cuda)
+
+    def run(rows, tokens, out):
+        a2a = AllToAll(k, E, H, T, None)
+        excl = torch.empty((E + 1,), dtype=torch.int32, device=cuda)
+        a2a.dispatch(excl, rows, tokens, idx, T)
+        got = rows[:int(excl[E])].clone()
+        a2a.combine(out, w, rows, T)
+        return got, out.clone()
+
+    def zeros():
+        return torch.zeros((T * k + T, H), dtype=torch.bfloat16, device=cuda)
+
+    want_rows, want_out = run(zeros()[:T * k], x, torch.empty_like(x))
+    both = zeros()   # the rows are written over the tokens (which the identity experts of the combine read: not compared)
+    both[:T] = x
+    assert torch.equal(run(both[:T * k], both[:T], torch.empty_like(x))[0], want_rows)
+    rows = zeros()[:T * k]
+    got, out = run(rows, x, rows[:T])
+    assert torch.equal(got, want_rows) and torch.equal(out, want_out)
+    a2a = AllToAll(k, E, H, T, None)
+    a2a.dispatch(torch.empty((E + 1,), dtype=torch.int32, device=cuda), zeros()[:T * k], x, idx, T)
+    flat = zeros().view(-1)
+    for target in (torch.empty_like(x), flat[1:1 + T * H].view(T, H)):
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            a2a.combine(target, w, flat[1:1 + T * k * H].view(T * k, H), T)
+    with pytest.raises(RuntimeError, match="rows of 512 bytes"):
+        a2a.combine(torch.empty_like(x), w, torch.zeros((T * k, H), device=cuda), T)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("D", [256, 512])
 def test_fast_oep_ops(cuda, eps_pkg, D):
     """Lookups in a (here one-rank) sharded table: out[i] = table[id_i], negative ids leave their rows untouched; with
