@@ -149,16 +149,12 @@ template <int kCtas>
 __global__ void __launch_bounds__(kThreads, 1)
 grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                          const Params p) {
-  // Used as it stands (not through a rounded-up address), so that the compiler knows every access for one to shared
-  // memory; the swizzle needs the 1024-byte alignment, which the check makes sure of.
+  // Used as it stands (see the FP8 kernel); the 1024-byte alignment that the swizzle needs is declared here, and
+  // configure_smem makes sure on the host that nothing lies before this array.
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using St = Storage<kCtas>;
   constexpr int kStages = St::kStages;
   St* sm = reinterpret_cast<St*>(smem_raw);
-  if ((smem_u32(smem_raw) & 1023u) != 0) {   // the same in every CTA
-    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, 51);
-    return;
-  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = kCtas == 2 ? cluster_ctarank() : 0u;   // 0 = the CTA that issues the MMAs
 
@@ -427,14 +423,14 @@ template <int kCtas>
 int launch_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int64_t tiles_max, int sm_count,
                 cudaStream_t st) {
   const size_t smem = sizeof(Storage<kCtas>);
+  static_assert(sizeof(Storage<kCtas>) <= kMaxSmem, "shared memory of one CTA");
   static std::atomic<int> max_units[64];   // per device: 0 = not configured yet, else CTAs (or pairs) that fit at once
   int dev = 0;
   cudaGetDevice(&dev);
   int fit = (dev >= 0 && dev < 64) ? max_units[dev].load(std::memory_order_acquire) : 0;
   if (fit == 0) {
-    cudaError_t e = cudaFuncSetAttribute(grouped_gemm_bf16_kernel<kCtas>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return fail(EPSB_ERR_CUDA, "cudaFuncSetAttribute(gemm bf16): %s", cudaGetErrorString(e));
+    const int rc = configure_smem(grouped_gemm_bf16_kernel<kCtas>, smem, "gemm bf16");
+    if (rc) return rc;
     fit = gemm_cta_limit(0);
     if (kCtas == 2) {
       // how many PAIRS the device can hold at once (a pair needs two SMs of one cluster-capable group)
@@ -450,7 +446,7 @@ int launch_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, i
       q.attrs = a;
       q.numAttrs = 1;
       int clusters = 0;
-      e = cudaOccupancyMaxActiveClusters(&clusters, grouped_gemm_bf16_kernel<kCtas>, &q);
+      const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, grouped_gemm_bf16_kernel<kCtas>, &q);
       if (e != cudaSuccess || clusters <= 0)
         return fail(EPSB_ERR_CUDA, "cudaOccupancyMaxActiveClusters(gemm bf16 pairs): %s", cudaGetErrorString(e));
       fit = clusters;

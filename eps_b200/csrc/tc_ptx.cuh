@@ -9,6 +9,25 @@
 namespace epsb {
 
 constexpr uint64_t kWaitLimitNs = 2000000000ull;
+constexpr size_t kMaxSmem = 232448;   // bytes of shared memory one CTA can have
+
+// Opts a kernel in to `smem` bytes of dynamic shared memory, and refuses one whose dynamic array cannot start at a multiple
+// of 1024 bytes (what the 128-byte swizzle needs): it lies behind what the system reserves and the kernel's static arrays.
+template <class Kernel>
+inline int configure_smem(Kernel* kernel, size_t smem, const char* what) {
+  int dev = 0, reserved = 0;
+  cudaFuncAttributes attr = {};
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, kernel);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return fail(EPSB_ERR_CUDA, "shared memory of %s: %s", what, cudaGetErrorString(e));
+  EPSB_REQUIRE((reserved + attr.sharedSizeBytes) % 1024 == 0, EPSB_ERR_CUDA,
+               "%s: its shared memory starts %zu bytes into the CTA's, not at a multiple of 1024", what,
+               (size_t)reserved + attr.sharedSizeBytes);
+  return EPSB_OK;
+}
+
 // Shared-memory matrix descriptor (K-major, SWIZZLE_128B), high word: stride-byte-offset 1024 B (8 rows x 128 B)
 // >> 4 = 64, descriptor version 1 (bits 46-47), layout SWIZZLE_128B = 2 (bits 61-63).
 constexpr uint32_t kDescHi = 64u | (1u << 14) | (2u << 29);

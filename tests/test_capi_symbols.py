@@ -55,6 +55,19 @@ def test_fastep_reduce_refuses_misaligned_rows():
             call("epsb_fastep_reduce", rows, raw, shared, a, a, 4, 2, 256, out, None)
 
 
+def test_gemm_kernels_have_no_static_shared_memory():
+    """The GEMM kernels use their dynamic shared memory from its first byte, which is 1024-byte aligned as long as no static
+    array lies before it (the host refuses the launch otherwise): what ptxas said when they were built."""
+    from eps_b200 import build
+
+    names = ("grouped_gemm", "grouped_gemm_bf16")
+    logs = [os.path.join(build.OBJ_DIR, n + ".ptxas.log") for n in names]
+    build.build(force=not all(os.path.exists(p) for p in logs))
+    for p in logs:
+        used = [line for line in open(p) if "Used" in line and "registers" in line]
+        assert len(used) >= 2 and not any("smem" in line for line in used), (p, used)
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     import pytest
 
