@@ -459,8 +459,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ AMaps tmap_a, const __grid_const
         return (uint32_t)(128 * half + ch * 32);
       };
       auto tmem_of = [&](uint32_t k_it) -> uint32_t { return lane_addr + (k_it & 1u) * (uint32_t)kBN; };
-      auto wait_full = [&](bool ready) -> bool {
-        bool good = ready || mbar_wait(&sm->empty[pos.stage], pos.phase, sm, p.status, 31);
+      auto wait_full = [&]() -> bool {
+        bool good = mbar_wait(&sm->empty[pos.stage], pos.phase, sm, p.status, 31);
         pos.next();
         good = __all_sync(0xffffffffu, good);
         if (good) tc_fence_after();
@@ -472,17 +472,16 @@ grouped_gemm_fp8_kernel(const __grid_constant__ AMaps tmap_a, const __grid_const
       // flight).  The chain crosses K steps: once the fourth load of a step has landed the buffer is released to
       // the MMA warp, the first load of the NEXT step is issued, and only then is the fourth chunk folded.
       // Two 32-register landing arrays beside the 128 accumulators: no spills at 232 registers.
+      // Whether the next step is ready is not asked before this one is drained: try_wait may suspend the warp, and its late
+      // release then holds up the MMAs (gate/up 32 x 1024 1.53 ms with it, 1.10 without; down 0.623, 0.605), and test_wait,
+      // which does not suspend, gains nothing either (1.17; 0.609).
       uint32_t t0[32], t1[32];
-      ok = wait_full(false);
+      ok = wait_full();
       if (!ok) break;
       tmem_ld32_async(tmem_of(it) + col_of(0), t0);
       for (int kb = 0; kb < KB; kb++, it++) {
         s0 = sa * sb0;
         s1 = sa * sb1;
-        // Asked now, used once this step has landed: where the drain is behind the MMAs the answer is there by then.  Not
-        // in gate/up mode, where the two K-step scales leave no register for it: measured at 32 experts x 1024 rows 1.48 ms
-        // with the question and 1.10 without, down 0.64 ms with and 0.67 without.
-        const bool ready = kMode != EPSB_GEMM_GATEUP && kb + 1 < KB && mbar_try(&sm->empty[pos.stage], pos.phase);
         if (kb + 1 < KB) {
           sa = __ldg(as_row + kb + 1);
           sb0 = __ldg(bs0 + kb + 1);
@@ -507,7 +506,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ AMaps tmap_a, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm->tmem_empty[it & 1u]);
         if (kb + 1 < KB) {
-          ok = wait_full(ready);
+          ok = wait_full();
           if (!ok) break;
           tmem_ld32_async(tmem_of(it + 1) + col_of(0), t0);
         }
