@@ -149,6 +149,8 @@ class MoELayerFP8:
 
         def stage_gemms(s):
             ex = excl[s * eps_:(s + 1) * eps_ + 1]
+            if self.direct_sources and not self.gemm_gathers_rows:   # one gather from the source rows into expert order
+                sched.gather_gemm_rows(expert_weights, xq, xs, self.A[:D], self.A_s[:D], row_w, s)
             ev = self.gateup_events if s == 0 else None
             if ev is not None:
                 ev[0].record()
@@ -157,8 +159,6 @@ class MoELayerFP8:
                                      self.wgu_s[s * eps_:(s + 1) * eps_], ex, out=self.act[:D],
                                      out_scales=self.act_s[:D], status=self.status, a_rows=a_rows[:D])
             else:
-                if self.direct_sources:   # one gather from the source rows into expert order
-                    sched.gather_gemm_rows(expert_weights, xq, xs, self.A[:D], self.A_s[:D], row_w, s)
                 ops.grouped_gemm_fp8(ops.GEMM_GATEUP, self.A[:D], self.A_s[:D], self.wgu[s * eps_:(s + 1) * eps_],
                                      self.wgu_s[s * eps_:(s + 1) * eps_], ex, out=self.act[:D],
                                      out_scales=self.act_s[:D], status=self.status)

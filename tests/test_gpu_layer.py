@@ -220,3 +220,30 @@ def test_forward_host_matches_forward(cuda, oracle):
     for o, (x, idx, w) in zip(outs_h, wants):
         ref = layer.forward(x.to(cuda), idx.to(cuda), w.to(cuda))
         assert torch.equal(o, ref.cpu())
+
+
+def test_gateup_events_enclose_the_gemm_alone(cuda, oracle, monkeypatch):
+    """What the events around the gate/up GEMM measure: the GEMM of the first stage, not the gather of its rows."""
+    from eps_b200 import ops, workloads
+    from eps_b200.layer import MoELayerFP8
+
+    T, H, I, E, k = 16, 256, 128, 4, 2
+    cfg = workloads.CONFIGS[0].scaled(tokens_per_rank=T, hidden=H, inter=I, num_experts=E, top_k=k)
+    dev_w, _ = _weights(cfg, range(E), cuda, oracle)
+    layer = MoELayerFP8(H, I, E, k, T, *dev_w, num_stages=2)
+    seen = []
+
+    def logged(name, fn):
+        return lambda *a, **kw: (seen.append(name), fn(*a, **kw))[1]
+
+    class Mark:
+        def __init__(self, name):
+            self.record = lambda: seen.append(name)
+
+    monkeypatch.setattr(ops, "grouped_gemm_fp8", logged("gemm", ops.grouped_gemm_fp8))
+    monkeypatch.setattr(layer.sched, "gather_gemm_rows", logged("gather", layer.sched.gather_gemm_rows))
+    layer.gateup_events = (Mark("start"), Mark("end"))
+    idx, w = workloads.make_routing(cfg)
+    layer.forward(workloads.make_tokens(cfg).to(cuda), idx.to(cuda), w.to(cuda))
+    torch.cuda.synchronize()
+    assert seen == ["gather", "start", "gemm", "end", "gemm", "gather", "gemm", "gemm"]
