@@ -1,11 +1,13 @@
 // Weighted row reductions of the combine path and the unfused SwiGLU (sm_100a).
 //
 // A warp owns an output row, or one of `parts` interleaved parts of it when there are too few rows to fill the chip
-// (row_parts below); each lane walks it in 16-byte vectors (8 bf16)
+// (row_parts, fill_parts below); each lane walks it in 16-byte vectors (8 bf16)
 // and issues the loads of all summands of a vector before accumulating, so k
 // (or W) independent 16-byte loads per lane are in flight.  Two arithmetic
 // families are provided: "_ref" reproduces the reference kernels' bf16
 // multiply/accumulate order; the others accumulate in fp32 and round once.
+#include <climits>
+
 #include "common.cuh"
 
 namespace epsb {
@@ -16,6 +18,10 @@ constexpr int kRedThreads = 256;
 constexpr int kRedWarps = kRedThreads / 32;
 constexpr int kMaxSlots = 16;  // largest top-k / world size a register-resident kernel takes
 // Kernels are instantiated for 4, 8, 12 and 16 summands: fewer registers -> more resident warps -> more loads in flight.
+// CTAs that are resident on an SM at once, by the summands (the loads in flight are registers); row_parts counts on it.
+// Without the bound 12 summands take 134 registers, one CTA (2400 rows of 1024 21.5 us instead of 13.5), and 16 up to 192
+// (1200 rows of 7168 69 us instead of 50).
+constexpr int red_ctas(int slots) { return slots <= 4 ? 4 : (slots <= 8 ? 3 : 2); }
 
 union BfVec {
   uint4 u;
@@ -67,7 +73,7 @@ struct StageWindows {
 // ---------------------------------------------------------------- local reduce (expert rank)
 
 template <bool kRefArith, int kSlots>
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, red_ctas(kSlots))
 local_reduce_kernel(const uint8_t* __restrict__ y, const float* __restrict__ w_recv,
                     const int32_t* __restrict__ scale_map, const int32_t* __restrict__ red_map, StageWindows win,
                     int k, int64_t H, int parts, uint8_t* __restrict__ send) {
@@ -142,7 +148,7 @@ local_reduce_kernel(const uint8_t* __restrict__ y, const float* __restrict__ w_r
 // (the return row of token t; with one rank the return buffer IS the collect buffer).  fp32 accumulation in
 // slot order, one rounding.  Replaces local_reduce -> (no-op exchange) -> global_reduce for ep_world_size 1.
 template <int kSlots>
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, red_ctas(kSlots))
 reduce_ep1_kernel(const uint8_t* __restrict__ y, const int32_t* __restrict__ red_map,
                   const int32_t* __restrict__ glob_map, const int32_t* __restrict__ ret_incl, int S,
                   const uint8_t* __restrict__ shared, const uint8_t* __restrict__ x,
@@ -190,7 +196,7 @@ reduce_ep1_kernel(const uint8_t* __restrict__ y, const int32_t* __restrict__ red
 // ---------------------------------------------------------------- global reduce (source rank)
 
 template <bool kRefArith, int kSlots>
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, red_ctas(kSlots))
 global_reduce_kernel(const uint8_t* __restrict__ recv, const int32_t* __restrict__ glob_map,
                      const uint8_t* __restrict__ shared, const uint8_t* __restrict__ x,
                      const float* __restrict__ zero_scale, int T, int W, int64_t H, int parts, uint8_t* __restrict__ out) {
@@ -328,7 +334,7 @@ global_reduce_wide_kernel(const uint8_t* __restrict__ recv, const int32_t* __res
 // ---------------------------------------------------------------- fast_ep combine
 
 template <int kSlots>
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, red_ctas(kSlots))
 fastep_reduce_kernel(const uint8_t* __restrict__ rows_in, const uint8_t* __restrict__ raw,
                      const uint8_t* __restrict__ shared, const float* __restrict__ w,
                      const int32_t* __restrict__ mapping, int T, int k, int64_t H, int parts, uint8_t* __restrict__ out) {
@@ -411,13 +417,29 @@ silu_kernel(const uint8_t* __restrict__ gate_up, uint8_t* __restrict__ act, cons
     else { constexpr int kS = 16; __VA_ARGS__; }                \
   } while (0)
 
-// Parts of a row of H bf16: 1 where the rows alone fill every SM with warps, else as many as do, down to one 16-byte vector
-// per lane.  A warp alone walks a 7168-wide row with 8 summands in 28 dependent steps of one memory latency: 128 rows took
-// 36 us undivided (0.5 TB/s) where the bytes need 3.
-int row_parts(int64_t rows, int64_t H) {
-  const int64_t steps = (H / 8 + 31) / 32;
-  const int64_t want = (int64_t)sm_count() * 8 * kRedWarps / (rows > 0 ? rows : 1);
+// Parts of a row of H bf16 where a lane has few loads in flight (SwiGLU, the reduction over many ranks): as many as keep 64
+// warps an SM busy, down to one 16-byte vector per lane.
+int fill_parts(int64_t rows, int64_t H) {
+  const int64_t steps = (H / 8 + 31) / 32, want = (int64_t)sm_count() * 8 * kRedWarps / (rows > 0 ? rows : 1);
   return (int)(want < 1 ? 1 : (want > steps ? steps : want));
+}
+
+// Parts of a row where a lane has a vector of every summand in flight, so that few rows fill the chip.  A warp alone walks a
+// 7168-wide row in 28 dependent steps of one memory latency, and spends about two more on the row's indices and weights;
+// warps that are not resident at once wait for others.  Taken is the division with the fewest steps in a row, the coarsest
+// of equals (two parts where whole rows need a second wave); past 4/3 of the resident warps rows stay whole.  Device us with 8 summands (fast_ep), undivided / fill_parts /
+// so: 300 rows of 7168 16.0 / 7.4 / 6.4, 1200 of 1024 5.1 / 5.3 / 4.5, 2400 of 4096 21 / 27 / 21, 4000 of 7168 83 / 74 / 72 (ranks).
+int row_parts(int64_t rows, int64_t H, int slots) {
+  const int steps = (int)((H / 8 + 31) / 32), resident = sm_count() * red_ctas(slots) * kRedWarps;
+  if (3 * rows > 4ll * resident) return 1;
+  int best = 1, least = INT_MAX;
+  for (int p = 1; p <= steps; p++) {
+    const int waves = ((int)rows * p + resident - 1) / resident;
+    const int cost = waves * ((steps + p - 1) / p + 2);
+    if (cost < least || (cost == least && p == 2 && rows > resident)) least = cost, best = p;
+    if (waves > 8) break;
+  }
+  return best;
 }
 
 int red_grid(int64_t rows) {
@@ -450,7 +472,8 @@ extern "C" int epsb_local_reduce_ref(const void* y, const float* w_recv, const i
   EPSB_REQUIRE(stage >= -1 && stage < S, EPSB_ERR_INVALID, "stage %d out of range for %d stages", stage, S);
   if (max_rows <= 0) return EPSB_OK;
   StageWindows win{ret_incl, W, S, stage};
-  const int parts = row_parts(stage < 0 ? max_rows : (max_rows + S - 1) / S, H);   // a stage covers about 1/S of the rows
+  const int64_t rows = stage < 0 ? max_rows : (max_rows + S - 1) / S;   // a stage covers about 1/S of them
+  const int parts = row_parts(rows, H, k);
   EPSB_SLOT_SWITCH(k, (local_reduce_kernel<true, kS><<<red_grid(max_rows * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       (const uint8_t*)y, w_recv, scale_map, red_map, win, k, H, parts, (uint8_t*)send)));
   return check_launch("local_reduce_ref");
@@ -464,7 +487,8 @@ extern "C" int epsb_local_reduce(const void* y, const int32_t* red_map, const in
   EPSB_REQUIRE(stage >= -1 && stage < S, EPSB_ERR_INVALID, "stage %d out of range for %d stages", stage, S);
   if (max_rows <= 0) return EPSB_OK;
   StageWindows win{ret_incl, W, S, stage};
-  const int parts = row_parts(stage < 0 ? max_rows : (max_rows + S - 1) / S, H);   // a stage covers about 1/S of the rows
+  const int64_t rows = stage < 0 ? max_rows : (max_rows + S - 1) / S;   // a stage covers about 1/S of them
+  const int parts = row_parts(rows, H, k);
   EPSB_SLOT_SWITCH(k, (local_reduce_kernel<false, kS><<<red_grid(max_rows * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       (const uint8_t*)y, nullptr, nullptr, red_map, win, k, H, parts, (uint8_t*)send)));
   return check_launch("local_reduce");
@@ -479,7 +503,7 @@ static int launch_global_reduce(const void* recv, const int32_t* glob_map, const
   EPSB_REQUIRE(zero_scale == nullptr || x != nullptr, EPSB_ERR_INVALID, "zero_scale needs the raw input x");
   if (T <= 0) return EPSB_OK;
   auto st = static_cast<cudaStream_t>(stream);
-  const int parts = row_parts(T, H);
+  const int parts = W <= kMaxSlots ? row_parts(T, H, W) : fill_parts(T, H);
   if (W <= kMaxSlots)
     EPSB_SLOT_SWITCH(W, (global_reduce_kernel<kRef, kS><<<red_grid((int64_t)T * parts), kRedThreads, 0, st>>>(
         (const uint8_t*)recv, glob_map, (const uint8_t*)shared, (const uint8_t*)x, zero_scale, T, W, H, parts, (uint8_t*)out)));
@@ -509,7 +533,7 @@ extern "C" int epsb_reduce_ep1(const void* y, const int32_t* red_map, const int3
   EPSB_REQUIRE(S > 0, EPSB_ERR_INVALID, "num_stages %d", S);
   EPSB_REQUIRE(zero_scale == nullptr || x != nullptr, EPSB_ERR_INVALID, "zero_scale needs the raw input x");
   if (T <= 0) return EPSB_OK;
-  const int parts = row_parts(T, H);
+  const int parts = row_parts(T, H, k);
   EPSB_SLOT_SWITCH(k, (reduce_ep1_kernel<kS><<<red_grid((int64_t)T * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       (const uint8_t*)y, red_map, glob_map, ret_incl, S, (const uint8_t*)shared, (const uint8_t*)x, zero_scale, T, k, H,
       parts, (uint8_t*)out)));
@@ -526,7 +550,7 @@ extern "C" int epsb_fastep_reduce(const void* rows, const void* raw, const void*
   if (T <= 0) return EPSB_OK;
   EPSB_REQUIRE(vec_aligned(raw) && vec_aligned(shared) && vec_aligned(out), EPSB_ERR_INVALID,
                "row buffers must be 16-byte aligned");
-  const int parts = row_parts(T, H);
+  const int parts = row_parts(T, H, k);
   EPSB_SLOT_SWITCH(k, (fastep_reduce_kernel<kS><<<red_grid((int64_t)T * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       (const uint8_t*)rows, (const uint8_t*)raw, (const uint8_t*)shared, w, mapping, T, k, H, parts, (uint8_t*)out)));
   return check_launch("fastep_reduce");
@@ -537,7 +561,7 @@ extern "C" int epsb_silu_run(const void* gate_up, void* act, const int32_t* excl
   EPSB_REQUIRE(inter_size > 0 && inter_size % 8 == 0, EPSB_ERR_INVALID, "Unsupported inter_size: %lld",
                (long long)inter_size);
   if (rows <= 0) return EPSB_OK;
-  const int parts = row_parts(rows, inter_size);
+  const int parts = fill_parts(rows, inter_size);
   silu_kernel<<<red_grid(rows * parts), kRedThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       (const uint8_t*)gate_up, (uint8_t*)act, exclusive_sum, num_experts, rows, inter_size, parts);
   return check_launch("silu_run");

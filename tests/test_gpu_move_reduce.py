@@ -294,6 +294,41 @@ def test_a_rows_sum_does_not_depend_on_how_many_rows_there_are(cuda, H):
         assert torch.equal(part, full[:n]), n
 
 
+@pytest.mark.parametrize("slots", [3, 8, 11, 16, 20])
+@pytest.mark.parametrize("H", [8, 264, 2304])
+def test_reductions_do_not_depend_on_how_a_row_is_divided(cuda, H, slots):
+    """The same for every reduction and the SwiGLU, over row counts on both sides of each division: the first n rows of a
+    call with many rows are what a call with n rows gives (20 summands: only the reduction over ranks takes them)."""
+    from eps_b200 import ops
+
+    T = 2400
+    g = torch.Generator().manual_seed(H + slots)
+    src = torch.randn((2 * T, H), generator=g).to(torch.bfloat16).to(cuda)
+    x = torch.randn((T, H), generator=g).to(torch.bfloat16).to(cuda)
+    zs, w = torch.rand((T,), generator=g).to(cuda), torch.rand((T, slots), generator=g).to(cuda)
+    glob = torch.arange(T, dtype=torch.int32, device=cuda)
+    # the rows of output row t lie below (t + 1) * slots: in a call with n rows, entries of n * slots and more say "no row"
+    red = (torch.rand((T, slots), generator=g) * (torch.arange(T).unsqueeze(1) + 1) * slots).int().remainder(2 * T).to(cuda)
+
+    def run(n):
+        out = lambda: torch.full((n, H), 7.0, dtype=torch.bfloat16, device=cuda)
+        red_n, incl = red[:n].contiguous().view(-1), torch.tensor([n], dtype=torch.int32, device=cuda)
+        got = [ops.global_reduce(src, red_n, out(), slots, x=x, zero_scale=zs, ref_arith=ref)
+               for ref in (False, True)]
+        if slots <= 16:
+            got.append(ops.reduce_ep1(src, red_n, glob, incl, 1, slots, out(), shared=x, x=x, zero_scale=zs))
+            got.append(ops.local_reduce(src, red_n, incl, slots, 1, 1, -1, out()))
+            got.append(ops.local_reduce_ref(src, w, glob, red_n, incl, slots, 1, 1, -1, out()))
+            got.append(ops.fastep_reduce(src, x, w[:n].contiguous(), red_n, out(), shared=x))
+        got.append(ops.silu_run(src.view(T, 2 * H)[:n], out()))
+        return got
+
+    full = run(T)
+    for n in (1, 90, 300, 700, 1000, 1200, 1300, 1700):
+        for i, (a, b) in enumerate(zip(run(n), full)):
+            assert torch.equal(a, b[:n]), (n, i)
+
+
 @pytest.mark.parametrize("n_seg", [1, 255, 256, 257, 1024, 1100])
 def test_arrange_rows_segment_counts(cuda, n_seg):
     """Segments of 0 to 5 rows, copied to another order, around the number of segments a CTA scans at a time."""
