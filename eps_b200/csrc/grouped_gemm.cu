@@ -326,9 +326,10 @@ grouped_gemm_fp8_kernel(const __grid_constant__ AMaps tmap_a, const __grid_const
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == 0) {
-      // ------------------------------------------------ TMA producer.  Lane 0 waits for the stage, announces the
-      // bytes and loads the weights; the A tile comes either as one box load (lane 0) or, when the caller gave a
-      // row index per GEMM row, as one gather4 per lane (lane j brings tile rows 4j .. 4j+3).
+      // ------------------------------------------------ TMA producer.  The warp waits for the stage together;
+      // one elected lane announces the bytes and loads the weights.  The A tile comes either as one box load (the same
+      // lane) or, when the caller gave a row index per GEMM row, as one gather4 per lane (lane j brings tile rows 4j ..
+      // 4j+3).
       const int KB = p.kb, total_tiles = tile_count();
       const bool gather = p.a_rows != nullptr;
       RingPos<kStages> pos;

@@ -418,7 +418,8 @@ silu_kernel(const uint8_t* __restrict__ gate_up, uint8_t* __restrict__ act, cons
   } while (0)
 
 // Parts of a row of H bf16 where a lane has few loads in flight (SwiGLU, the reduction over many ranks): as many as keep 64
-// warps an SM busy, down to one 16-byte vector per lane.
+// warps an SM busy, down to one 16-byte vector per lane.  `rows` is what the buffer holds: the window that a call with device
+// bounds works on may be shorter, and is then divided less than it could be.
 int fill_parts(int64_t rows, int64_t H) {
   const int64_t steps = (H / 8 + 31) / 32, want = (int64_t)sm_count() * 8 * kRedWarps / (rows > 0 ? rows : 1);
   return (int)(want < 1 ? 1 : (want > steps ? steps : want));

@@ -69,9 +69,7 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
-// Bounded wait.  Returns false when the CTA is aborting (this wait or another one gave up).  The first try stands alone
-// in the instruction stream: in the steady state of a pipeline it succeeds, and the roles that are one thread have to
-// get through a K step in few instructions.
+// The wait's loop, bounded.  Returns false when the CTA is aborting (this wait or another one gave up).
 template <class Storage>
 __device__ __forceinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, Storage* sm, int32_t* status, int code) {
   uint64_t t0 = 0;
@@ -93,6 +91,8 @@ __device__ __forceinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, S
     }
   }
 }
+// Bounded wait, by all lanes of a warp or by one.  The first try stands alone in the instruction stream: in the steady state
+// of a pipeline it succeeds, and the producer and MMA warps have to get through a K step in few instructions.
 template <class Storage>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, Storage* sm, int32_t* status, int code) {
   if (__builtin_expect(mbar_try(bar, parity) != 0, 1)) return true;

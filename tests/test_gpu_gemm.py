@@ -152,6 +152,30 @@ def test_gemm_gateup_activation_in_every_binade(cuda, oracle, rows):
     assert np.all(q.cpu().numpy() == top)
 
 
+@pytest.mark.parametrize("rows", [128, 40, 7])
+def test_gemm_gateup_group_whose_reciprocal_scale_overflows(cuda, oracle, rows):
+    """Activations around 2^-126: amax/448 is subnormal and its reciprocal infinite, so act * inv is +inf, -inf or (for a
+    zero) a NaN, and the codes are 448, -448 and 448."""
+    from eps_b200 import ops
+
+    I, K = 128, 128
+    one = int(np.flatnonzero(oracle.e4m3_table() == 1.0)[0])
+    A, B = np.zeros((rows, K), dtype=np.uint8), np.zeros((1, 2 * I, K), dtype=np.uint8)
+    A[:, 5] = one
+    B[:, :I, 5] = one
+    sign = np.arange(I) % 3 - 1
+    B[0, I:, 5] = np.where(sign == 0, 0, np.where(sign < 0, 0x80 | one, one))
+    b_s = np.array([1.0, 2.0 ** -125], dtype=np.float32).reshape(1, 2, 1)
+    status = torch.zeros(4, dtype=torch.int32, device=cuda)
+    q, s = ops.grouped_gemm_fp8(ops.GEMM_GATEUP, _dev(A, cuda), torch.ones((rows, 1), device=cuda), _dev(B, cuda),
+                                _dev(b_s, cuda), torch.tensor([0, rows], dtype=torch.int32, device=cuda), status=status)
+    torch.cuda.synchronize()
+    _check_status(status)
+    want = 2.0 ** -125 / (1.0 + np.exp(-1.0)) / 448.0
+    assert np.all(np.abs(s.cpu().numpy() - want) <= 2.0 ** -21 * want + 2.0 ** -149)   # a subnormal, a multiple of 2^-149
+    assert np.array_equal(q.cpu().numpy(), np.tile(np.where(sign < 0, 0xFE, 0x7E).astype(np.uint8), (rows, 1)))
+
+
 @pytest.mark.parametrize("rows,N,K", [([128], 256, 128), ([9, 250, 0, 40], 512, 1408 - 1408 % 128),
                                        ([130, 64, 33, 1, 161], 384, 256)])
 def test_gemm_down_weighted(cuda, oracle, rows, N, K):

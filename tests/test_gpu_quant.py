@@ -28,6 +28,29 @@ def test_quant_1x128_bit_exact(cuda, oracle, rows, cols, div_mode):
     assert np.array_equal(q.cpu().numpy(), rq)
 
 
+@pytest.mark.parametrize("div_mode", [0, 1])
+def test_quant_groups_whose_reciprocal_scale_overflows(cuda, oracle, div_mode):
+    """amax/448 below 2^-128: the reciprocal is infinite, so x * inv is +inf, -inf or (for a zero) a NaN; also the groups
+    around that line and, for weights, the same in a block."""
+    from eps_b200 import ops
+
+    g = torch.Generator().manual_seed(17)
+    x = torch.randn((24, 384), generator=g)
+    x[:, ::7] = 0
+    amax = x.view(24, 3, 128).abs().amax(-1, keepdim=True)
+    top = 448.0 * 2.0 ** -128 * torch.logspace(-2, 1, 72).view(24, 3, 1)   # 1e-2 .. 10 times the line
+    x = (x.view(24, 3, 128) / amax * top).view(24, 384).to(torch.bfloat16)
+    q, s = ops.per_token_group_quant_fp8(x.to(cuda), div_mode=div_mode)
+    rq, rs = oracle.quant_1x128(_bits(x), div_mode=div_mode)
+    assert np.array_equal(s.cpu().numpy().view(np.uint32), rs.view(np.uint32))
+    assert np.array_equal(q.cpu().numpy(), rq)
+    assert (rq == 0xFE).sum() > 100 and (rq == 0x7E).sum() > 100
+    w = x[:1].expand(128, 384).contiguous().unsqueeze(0)
+    q, s = ops.quant_block128(w.to(cuda))
+    rq, rs = oracle.quant_block128(w.to(torch.float32).numpy())
+    assert np.array_equal(s.cpu().numpy().view(np.uint32), rs.view(np.uint32)) and np.array_equal(q.cpu().numpy(), rq)
+
+
 def test_quant_empty_and_errors(cuda):
     from eps_b200 import ops
     from eps_b200._lib import EpsError
